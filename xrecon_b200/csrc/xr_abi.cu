@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "xr_cell_tma.cuh"
+#include "xr_dd2d.cuh"
 #include "xr_vox_prefix.cuh"
 #include "xr_vox_stage.cuh"
 #include "xr_ragged.cuh"
@@ -130,7 +131,23 @@ Geom geom_from(const xr_geom2d* p) {
 struct Layout {
     size_t hdr, bA, bB, colQ, colR, colE, colF, colM, arc, colWR, volT, volR, volF, sinoS, pfxF, total;
     bool has_arc, has_pfx;
+    // 2D batches: the interleaved copy of the input, il_groups groups of il_nb
+    // images at a time (il_nb = 1: none); `total` without it is `base`
+    size_t il, base;
+    int il_nb, il_groups;
+    // 2D pixel gathers of up to PT_MAX_BATCH images: the row tables and their
+    // flags (0: none)
+    size_t tab, flags;
 };
+
+// 2D batches share each cell's or pixel's geometry over NB images, whose
+// input is interleaved first (xr_dd2d.cuh): NB is the batch rounded up to 2, 4
+// or 8.  Inputs whose group of NB would take more than 1 GiB are not
+// interleaved; the copy holds at most 256 MiB of groups (at least one), and
+// larger batches go through it in turns.  The pixel gathers take row tables up
+// to PT_MAX_BATCH images (if they fit IL_GROUP_MAX) and NB = 8 above.
+constexpr size_t IL_GROUP_MAX = (size_t)1 << 30, IL_MAX = (size_t)256 << 20;
+int interleave_nb(int nbatch) { return nbatch >= 5 ? 8 : nbatch >= 3 ? 4 : nbatch; }
 
 // Voxel-driven operators on a circular arc detector walk chained float32
 // boundary angles, which need the per-boundary entries of ViewTables::arc.
@@ -330,6 +347,26 @@ Layout layout(int dim3d, int op, const Geom& g, int nbatch, int nview, int dtype
     if (l.has_pfx)
         o = align256(o + (size_t)((g.W + PS_T - 1) / PS_T) * ((g.H + PS_T - 1) / PS_T) *
                              ((g.D + PFX_R - 1) / PFX_R) * nbatch * sizeof(int));
+    l.base = l.il = o;
+    l.il_nb = l.il_groups = 1;
+    const bool image_in = op == OP_A || op == OP_BT || op == OP_BWT;
+    l.tab = l.flags = 0;
+    if (!dim3d && op >= 0 && !image_in && nbatch <= PT_MAX_BATCH) {
+        const size_t bytes = V * nbatch * (g.Nu + 2) * ROW_ENTRY_BYTES;
+        if (bytes <= IL_GROUP_MAX) {
+            l.tab = o;    o = align256(o + bytes + 512);  // three arrays, 256-byte aligned each
+            l.flags = o;  o = align256(o + V * nbatch * sizeof(int));
+        }
+    } else if (!dim3d && op >= 0 && nbatch > 1 && nview > 0) {
+        const int nb = interleave_nb(nbatch), groups = (nbatch + nb - 1) / nb;
+        // images are kept twice (rows, flipped columns)
+        const size_t group = (image_in ? 2 * (size_t)g.H * g.W : V * g.Nu) * nb * sizeof(float);
+        if (group <= IL_GROUP_MAX) {
+            l.il_nb = nb;
+            l.il_groups = (int)std::min<size_t>(groups, std::max<size_t>(1, IL_MAX / group));
+            o = align256(o + group * l.il_groups);
+        }
+    }
     l.total = o;
     return l;
 }
@@ -830,66 +867,136 @@ int run3d(int op, const Geom& g, const TI* in, TO* out, const float* ang, int nb
     return check_cuda("vox_gather3d");
 }
 
-template <typename TI, typename TO>
-int run2d(int op, const Geom& g, const TI* in, TO* out, const float* ang, int nbatch, int nview,
-          char* ws, const Layout& l, cudaStream_t st, float oscale) {
-    const ViewTables vt = tables_at(ws, l);
+// Smallest power of two up to 8 by which splitting `warps` warps' loops of
+// `len` steps gives every SM four rounds of 48 warps: below that the gathers
+// wait on their own serial loops (one 720-view FBP of 256 x 256 pixels: 1006
+// us unsplit), above it a split only adds its reduction.
+int split2d(double warps, int len) {
+    int s = 1;
+    while (s < 8 && warps * s < 148.0 * 48 * 4 && 4 * s <= len) s *= 2;
+    return s;
+}
+
+// The three arrays of n row-table entries at p.
+RowTable row_table_at(char* p, size_t n) {
+    RowTable t;
+    t.q = reinterpret_cast<double2*>(p);
+    t.y = reinterpret_cast<float*>(p + align256(n * sizeof(double2)));
+    t.c = reinterpret_cast<float2*>(p + align256(n * sizeof(double2)) + align256(n * sizeof(float)));
+    return t;
+}
+
+template <typename TI, typename TG, int NB>
+int run2d_nb(int op, const Geom& g, const TI* in, void* out, int dto, const float* ang, int nbatch, int nview, char* ws,
+             const Layout& l, const ViewTables& vt, cudaStream_t st, float oscale) {
     const float cw = column_width(g, 0);
+    const Geom2F f = make_geom2f(g);
+    const bool image_in = op == OP_A || op == OP_BT || op == OP_BWT;
+    const long long n = image_in ? (long long)g.H * g.W : (long long)nview * g.Nu;
+    const int groups = (nbatch + NB - 1) / NB, per = NB == 1 ? groups : l.il_groups;
+    const TG *rows, *cols;
+    if constexpr (NB == 1) {
+        rows = in;
+        cols = reinterpret_cast<const TG*>(ws + l.volT);
+    } else {
+        rows = reinterpret_cast<const TG*>(ws + l.il);
+        cols = rows + per * n * NB;
+    }
+    for (int g0 = 0; g0 < groups; g0 += per) {
+        const int ng = std::min(per, groups - g0), b0 = g0 * NB;
+        const int nset = g0 == 0 ? nview * ((g.Nu + 1 + 255) / 256) : 0;
+        const int per_img = NB > 1 ? (int)((n + 255) / 256) : image_in ? ((g.W + 31) / 32) * ((g.H + 31) / 32) : 0;
+        prep2d_kernel<TI, NB><<<nset + ng * per_img, 256, 0, st>>>(
+            g, ang, nview, vt, nset, in + b0 * n, const_cast<TG*>(rows),
+            image_in ? const_cast<TG*>(cols) : nullptr, nbatch - b0, n, std::max(1, per_img));
+        if (int rc = check_cuda("prep2d")) return rc;
+        if (image_in) {
+            const int kb = (g.Nu + 31) / 32, LS = split2d((double)kb * nview * ng, std::min(g.W, g.H));
+            const dim3 grid((kb + 8 / LS - 1) / (8 / LS), nview, ng);
+            if (op == OP_A)
+                cell2d_kernel<TG, NB, OP_A><<<grid, 256, 0, st>>>(g, f, vt, rows, cols, out, dto, nview, b0, nbatch, cw, LS);
+            else if (op == OP_BT)
+                cell2d_kernel<TG, NB, OP_BT><<<grid, 256, 0, st>>>(g, f, vt, rows, cols, out, dto, nview, b0, nbatch, cw, LS);
+            else
+                cell2d_kernel<TG, NB, OP_BWT><<<grid, 256, 0, st>>>(g, f, vt, rows, cols, out, dto, nview, b0, nbatch, cw, LS);
+            if (int rc = check_cuda("cell2d")) return rc;
+        } else if constexpr (NB == 1 || NB == 8) {
+            const int tiles = pix2d_tiles(g.W, g.H), VS = split2d((double)tiles * ng, nview);
+            const dim3 grid((tiles + 8 / VS - 1) / (8 / VS), ng);
+            if (op == OP_AT)
+                pix2d_kernel<TG, NB, OP_AT><<<grid, 256, 0, st>>>(f, vt, rows, out, dto, nview, b0, nbatch, cw, oscale, VS);
+            else if (op == OP_B)
+                pix2d_kernel<TG, NB, OP_B><<<grid, 256, 0, st>>>(f, vt, rows, out, dto, nview, b0, nbatch, cw, oscale, VS);
+            else
+                pix2d_kernel<TG, NB, OP_BW><<<grid, 256, 0, st>>>(f, vt, rows, out, dto, nview, b0, nbatch, cw, oscale, VS);
+            if (int rc = check_cuda("pix2d")) return rc;
+        }
+    }
+    return XR_OK;
+}
+
+template <typename TI>
+int run2d(int op, const Geom& g, const TI* in, void* out, int dto, const float* ang, int nbatch, int nview, char* ws,
+          const Layout& l, cudaStream_t st, float oscale) {
     if (nview == 0) {
         if (op == OP_AT || op == OP_B || op == OP_BW) {
-            if (cudaMemsetAsync(out, 0, (size_t)g.H * g.W * nbatch * sizeof(TO), st) != cudaSuccess)
+            if (cudaMemsetAsync(out, 0, (size_t)g.H * g.W * nbatch * dtype_size(dto), st) != cudaSuccess)
                 return fail(XR_ERR_CUDA, "memset failed");
         }
         return XR_OK;
     }
-    {
-        dim3 grid((g.Nu + 1 + 127) / 128, nview);
-        setup_views_kernel<<<grid, 128, 0, st>>>(g, 0, ang, nview, vt);
-        if (int rc = check_cuda("setup_views")) return rc;
-    }
     if (nview > 65535 || nbatch > 65535) return fail(XR_ERR_UNSUPPORTED, "views or batch above 65535");
-    if (op == OP_A || op == OP_BT || op == OP_BWT) {
-        TI* imgT = reinterpret_cast<TI*>(ws + l.volT);
-        dim3 tg((g.W + 31) / 32, (g.H + 31) / 32, nbatch);
-        transpose_flip_kernel<TI><<<tg, dim3(32, 8), 0, st>>>(in, imgT, g.H, g.W, g.H);
-        if (int rc = check_cuda("transpose")) return rc;
-        dim3 grid((g.Nu + 127) / 128, nview, nbatch);
-        if (op == OP_A)
-            cell_gather2d_kernel<TI, TO, OP_A><<<grid, 128, 0, st>>>(g, vt, in, imgT, out, nview, cw);
-        else if (op == OP_BT)
-            cell_gather2d_kernel<TI, TO, OP_BT><<<grid, 128, 0, st>>>(g, vt, in, imgT, out, nview, cw);
-        else
-            cell_gather2d_kernel<TI, TO, OP_BWT><<<grid, 128, 0, st>>>(g, vt, in, imgT, out, nview, cw);
-        return check_cuda("cell_gather2d");
+    ViewTables vt = tables_at(ws, l);
+    // the pixel gathers' column steps take the place of colQ and colR, which
+    // 2D does not read (8 + 8 bytes per column)
+    vt.colQ = vt.colR = nullptr;
+    if (op == OP_AT || op == OP_B || op == OP_BW) vt.colWR = reinterpret_cast<float4*>(ws + l.colQ);
+    if (l.tab) {
+        const float cw = column_width(g, 0);
+        const Geom2F f = make_geom2f(g);
+        const RowTable tab = row_table_at(ws + l.tab, (size_t)nview * nbatch * (g.Nu + 2));
+        int* flags = reinterpret_cast<int*>(ws + l.flags);
+        if (op == OP_AT) table2d_kernel<TI, true><<<nview, 256, 0, st>>>(g, ang, nview, vt, in, nbatch, tab, flags);
+        else table2d_kernel<TI, false><<<nview, 256, 0, st>>>(g, ang, nview, vt, in, nbatch, tab, flags);
+        if (int rc = check_cuda("table2d")) return rc;
+        // View slices: first CTAs of a cluster (a CTA's warps then share each
+        // view's table in L1) until every SM holds four, what 64 registers a
+        // thread allow (720-view FBP of 256 x 256 pixels: 256 CTAs 276 us, 512
+        // CTAs 180 us); warps of a CTA only where that leaves SMs without work.
+        int CS = 1, VS = 1;
+        const int n1 = pix2t_ctas(g.W, g.H, 1) * nbatch;
+        while (CS < 8 && n1 * CS < 148 * 3 && 16 * CS <= nview) CS *= 2;
+        while (VS < 8 && (long long)pix2t_ctas(g.W, g.H, VS) * nbatch * CS < 148 && 8 * VS * CS <= nview) VS *= 2;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(pix2t_ctas(g.W, g.H, VS), nbatch, CS);
+        cfg.blockDim = dim3(256);
+        cfg.stream = st;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = CS;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        auto kern = op == OP_AT ? pix2t_kernel<TI, OP_AT> : op == OP_B ? pix2t_kernel<TI, OP_B> : pix2t_kernel<TI, OP_BW>;
+        if (cudaLaunchKernelEx(&cfg, kern, f, vt, tab, (const int*)flags, in, out, dto, nview, cw, oscale, VS) != cudaSuccess)
+            return check_cuda("pix2t (cluster launch)");
+        return check_cuda("pix2t");
     }
-    dim3 grid((g.W + 31) / 32, (g.H + 7) / 8, nbatch);
-    dim3 block(32, 8);
-    if (op == OP_AT)
-        vox_gather2d_kernel<TI, TO, OP_AT><<<grid, block, 0, st>>>(g, vt, in, out, nview, cw, oscale);
-    else if (op == OP_B)
-        vox_gather2d_kernel<TI, TO, OP_B><<<grid, block, 0, st>>>(g, vt, in, out, nview, cw, oscale);
-    else
-        vox_gather2d_kernel<TI, TO, OP_BW><<<grid, block, 0, st>>>(g, vt, in, out, nview, cw, oscale);
-    return check_cuda("vox_gather2d");
+    if (l.il_nb == 2) return run2d_nb<TI, float, 2>(op, g, in, out, dto, ang, nbatch, nview, ws, l, vt, st, oscale);
+    if (l.il_nb == 4) return run2d_nb<TI, float, 4>(op, g, in, out, dto, ang, nbatch, nview, ws, l, vt, st, oscale);
+    if (l.il_nb == 8) return run2d_nb<TI, float, 8>(op, g, in, out, dto, ang, nbatch, nview, ws, l, vt, st, oscale);
+    return run2d_nb<TI, TI, 1>(op, g, in, out, dto, ang, nbatch, nview, ws, l, vt, st, oscale);
 }
 
 template <typename TI>
 int dispatch_out(int dim3d, int op, const Geom& g, const void* in, void* out, int dto, const float* ang,
                  int nbatch, int nview, char* ws, const Layout& l, cudaStream_t st, float oscale) {
     const TI* i = static_cast<const TI*>(in);
-    if (dto == DT_F32) {
-        float* o = static_cast<float*>(out);
-        return dim3d ? run3d(op, g, i, o, ang, nbatch, nview, ws, l, st, oscale)
-                     : run2d(op, g, i, o, ang, nbatch, nview, ws, l, st, oscale);
-    }
-    if (dto == DT_BF16) {
-        __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out);
-        return dim3d ? run3d(op, g, i, o, ang, nbatch, nview, ws, l, st, oscale)
-                     : run2d(op, g, i, o, ang, nbatch, nview, ws, l, st, oscale);
-    }
-    __half* o = static_cast<__half*>(out);
-    return dim3d ? run3d(op, g, i, o, ang, nbatch, nview, ws, l, st, oscale)
-                 : run2d(op, g, i, o, ang, nbatch, nview, ws, l, st, oscale);
+    if (!dim3d) return run2d(op, g, i, out, dto, ang, nbatch, nview, ws, l, st, oscale);
+    if (dto == DT_F32) return run3d(op, g, i, static_cast<float*>(out), ang, nbatch, nview, ws, l, st, oscale);
+    if (dto == DT_BF16)
+        return run3d(op, g, i, static_cast<__nv_bfloat16*>(out), ang, nbatch, nview, ws, l, st, oscale);
+    return run3d(op, g, i, static_cast<__half*>(out), ang, nbatch, nview, ws, l, st, oscale);
 }
 
 int apply(int dim3d, int op, const Geom& g, const void* in, int dti, void* out, int dto, const float* ang,
@@ -901,11 +1008,15 @@ int apply(int dim3d, int op, const Geom& g, const void* in, int dti, void* out, 
     if ((!in && !(sino_in && nview == 0)) || (!out && !(!sino_in && nview == 0)))
         return fail(XR_ERR_INVALID_ARGUMENT, "null input or output pointer");
     if (nview > 0 && !ang) return fail(XR_ERR_INVALID_ARGUMENT, "null angles pointer");
-    const Layout l = layout(dim3d, op, g, nbatch, nview, dti);
-    if (!workspace || ws_bytes < l.total)
-        return fail(XR_ERR_WORKSPACE, "workspace of %zu bytes required, %zu given", l.total, ws_bytes);
+    Layout l = layout(dim3d, op, g, nbatch, nview, dti);
+    if (!workspace || ws_bytes < l.base)
+        return fail(XR_ERR_WORKSPACE, "workspace of %zu bytes required, %zu given", l.base, ws_bytes);
     if (reinterpret_cast<uintptr_t>(workspace) % 256 != 0)
         return fail(XR_ERR_WORKSPACE, "workspace must be 256-byte aligned");
+    // a scratch without room for the row tables or the interleaved copy
+    // (xr_dd2d_noalloc near its limit): the images' columns are walked one
+    // image at a time
+    if (ws_bytes < l.total) l.il_nb = l.il_groups = 1, l.tab = 0;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     char* ws = static_cast<char*>(workspace);
     if (dti == DT_F32) return dispatch_out<float>(dim3d, op, g, in, out, dto, ang, nbatch, nview, ws, l, st, oscale);
@@ -1131,7 +1242,7 @@ int helical(int op, const Geom& g, const HelOpts& o, const float* in, float* out
 
 struct RaggedLayout {
     size_t desc, sync;
-    std::vector<size_t> hdr, bA, bB, colQ, colR, colE, colF, colM, arc, imgT, filt;
+    std::vector<size_t> hdr, bA, bB, colWR, colE, colF, colM, arc, imgT, filt, tab, flags;
     size_t total;
 };
 
@@ -1160,8 +1271,7 @@ int ragged_tiles(const Geom& g, int nview, int list) {
     if (list == 0) return nview + (hw + 1023) / 1024;
     if (list == 1) return nview;
     if (list < 6) return nview * ((g.Nu + (32 << (list - 2)) - 1) / (32 << (list - 2)));
-    const int px = 256 / (1 << (list - 6));
-    return (hw + px - 1) / px;
+    return pix2t_ctas(g.W, g.H, 1 << (list - 6));
 }
 
 // Fixed device scratch of xr_dd2d_noalloc, the entry for callers that cannot
@@ -1422,7 +1532,7 @@ int xr_dd2d_noalloc(int op, const xr_geom2d* geom, const void* in, int dtype_in,
     if (int rc = xr::validate(g, 0, op, nbatch, nview)) return rc;
     if (!xr::dtype_ok(dtype_in) || !xr::dtype_ok(dtype_out))
         return xr::fail(XR_ERR_INVALID_ARGUMENT, "unsupported dtype (%d, %d)", dtype_in, dtype_out);
-    const size_t need = xr::layout(0, op, g, nbatch, nview, dtype_in).total;
+    const size_t need = xr::layout(0, op, g, nbatch, nview, dtype_in).base;
     if (need > (size_t)XR_NOALLOC_SCRATCH_BYTES)
         return xr::fail(XR_ERR_WORKSPACE,
                         "request needs %zu bytes of scratch; xr_dd2d_noalloc has a fixed %zu-byte scratch "
@@ -1549,8 +1659,7 @@ int xr_ragged2d_plan_create(const xr_ragged2d_instance* inst, int ninst, xr_ragg
         L.hdr.push_back(o);  o = align256(o + Vs * sizeof(ViewHdr));
         L.bA.push_back(o);   o = align256(o + Vs * (g.Nu + 1) * sizeof(double));
         L.bB.push_back(o);   o = align256(o + Vs * (g.Nu + 1) * sizeof(double));
-        L.colQ.push_back(o); o = align256(o + Vs * g.Nu * sizeof(double));
-        L.colR.push_back(o); o = align256(o + Vs * g.Nu * sizeof(double));
+        L.colWR.push_back(o); o = align256(o + Vs * g.Nu * sizeof(float4));
         L.colE.push_back(o); o = align256(o + Vs * g.Nu * sizeof(float));
         L.colF.push_back(o); o = align256(o + Vs * g.Nu * sizeof(float));
         L.colM.push_back(o); o = align256(o + Vs * g.Nu * sizeof(float));
@@ -1558,13 +1667,15 @@ int xr_ragged2d_plan_create(const xr_ragged2d_instance* inst, int ninst, xr_ragg
         if (g.type == GEO_ARC) o = align256(o + 2 * Vs * (g.Nu + 1) * sizeof(float4));  // Bw's chained walks
         L.imgT.push_back(o); o = align256(o + (size_t)g.H * g.W * sizeof(float));
         L.filt.push_back(o); o = align256(o + Vs * g.Nu * sizeof(float));
+        L.tab.push_back(o);  o = align256(o + Vs * (g.Nu + 2) * ROW_ENTRY_BYTES + 512);
+        L.flags.push_back(o); o = align256(o + Vs * sizeof(int));
     }
     for (int l = 0; l < 10; ++l) {
         if (tot[l] > 0x7fffffffll) { delete P; return fail(XR_ERR_UNSUPPORTED, "ragged batch too large"); }
         P->totals[l] = (int)tot[l];
     }
     L.total = o;
-    P->smem = std::max<size_t>(256, 3 * (size_t)P->max_nu + 16) * sizeof(float);
+    P->smem = std::max<size_t>(256 * P2 * P2, 3 * (size_t)P->max_nu + 16) * sizeof(float);
     if (P->smem > 200 * 1024) { delete P; return fail(XR_ERR_UNSUPPORTED, "detector too wide for the ragged kernel"); }
     if (cudaGetDevice(&P->device) != cudaSuccess) { delete P; return fail(XR_ERR_CUDA, "cudaGetDevice failed"); }
     if (P->smem > 48 * 1024 &&
@@ -1597,17 +1708,17 @@ int xr_ragged2d_plan_bind(xr_ragged2d_plan* P, const float* images, float* sino,
         const xr_ragged2d_instance& in = P->inst[i];
         RaggedDev& r = d[i];
         r.g = P->geom[i];
+        r.f = make_geom2f(r.g);
         r.vt.hdr = reinterpret_cast<ViewHdr*>(ws + L.hdr[i]);
         r.vt.bA = reinterpret_cast<double*>(ws + L.bA[i]);
         r.vt.bB = reinterpret_cast<double*>(ws + L.bB[i]);
-        r.vt.colQ = reinterpret_cast<double*>(ws + L.colQ[i]);
-        r.vt.colR = reinterpret_cast<double*>(ws + L.colR[i]);
+        r.vt.colQ = r.vt.colR = nullptr;
         r.vt.colE = reinterpret_cast<float*>(ws + L.colE[i]);
         r.vt.colF = reinterpret_cast<float*>(ws + L.colF[i]);
         r.vt.colM = reinterpret_cast<float*>(ws + L.colM[i]);
         r.vt.hel = nullptr;
         r.vt.arc = r.g.type == GEO_ARC ? reinterpret_cast<float4*>(ws + L.arc[i]) : nullptr;
-        r.vt.colWR = nullptr;
+        r.vt.colWR = reinterpret_cast<float4*>(ws + L.colWR[i]);
         r.nview = in.nview;
         r.cw = column_width(r.g, 0);
         r.scale = in.scale;
@@ -1615,6 +1726,8 @@ int xr_ragged2d_plan_bind(xr_ragged2d_plan* P, const float* images, float* sino,
         r.imgT = reinterpret_cast<float*>(ws + L.imgT[i]);
         r.sino = sino + in.sino_offset;
         r.filt_out = reinterpret_cast<float*>(ws + L.filt[i]);
+        r.tab = row_table_at(ws + L.tab[i], (size_t)in.nview * (r.g.Nu + 2));
+        r.flags = reinterpret_cast<int*>(ws + L.flags[i]);
         r.recon = recon + in.img_offset;
         r.ang = angles + in.ang_offset;
         r.filt = filt + in.filt_offset;

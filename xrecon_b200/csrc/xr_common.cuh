@@ -67,19 +67,22 @@ struct Geom {
 };
 
 // Per-view header (FP64 geometry, decisions taken like the reference CPU path).
-struct ViewHdr {
+// The first three 16-byte groups are what the 2D gathers read per view.
+struct alignas(16) ViewHdr {
     int use_x;      // common axis is x
     int keep;       // detector traversed in index order
     int nlines;     // H (use_x: lines are rows iy) or W (lines are columns ix)
     int npix;       // W or H: pixels along a line
+    float sf, cf;           // s and c in FP32
+    float sxr, syr;         // sx and sy rounded to FP32
+    float dcx, dcy;         // arc detector: central ray direction (column guesses)
+    float sxf, syf;         // the source as the reference holds it in float32
+    double q0, q1;          // 1 / Mv(L) = q0 + q1 * L   (1 for parallel)
     double beta, s, c;
     double sx, sy;          // source
     double spar, sperp;     // source coordinate along / across the axis
     double perpA, perpB;    // perpendicular coordinate of line L = perpA + perpB * L
-    double q0, q1;          // 1 / Mv(L) = q0 + q1 * L   (1 for parallel)
     double dpix;            // pixel size along the line (dx or dy)
-    float dcx, dcy;         // arc detector: central ray direction (column guesses)
-    float sxf, syf;         // the source as the reference holds it in float32
 };
 
 // Per-view tables, structure of arrays, view-major.
@@ -128,7 +131,8 @@ struct ViewTables {
     // k + 1 minus those of boundary k in FP32 (the column's width on line L
     // is dA + dB L pixels), and colR as a float pair.  The gather evaluates
     // one boundary and one colR per (pixel, view) in FP64 and steps to the
-    // neighbouring columns in FP32 from these.
+    // neighbouring columns in FP32 from these.  2D pixel gathers: {dA, dB,
+    // colE, 0}, in the memory of colQ and colR, which 2D does not read.
     float4* colWR;
 };
 
@@ -148,6 +152,14 @@ template <typename T> __device__ __forceinline__ void st(T* p, float v);
 template <> __device__ __forceinline__ void st<float>(float* p, float v) { *p = v; }
 template <> __device__ __forceinline__ void st<__nv_bfloat16>(__nv_bfloat16* p, float v) { *p = __float2bfloat16_rn(v); }
 template <> __device__ __forceinline__ void st<__half>(__half* p, float v) { *p = __float2half_rn(v); }
+
+// Hardware reciprocal (relative error 2^-23), one instruction: without the
+// denormal handling of __fdividef, whose operands here are lengths.
+__device__ __forceinline__ float rcp_fast(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
 
 // ---------------------------------------------------------------- geometry
 
@@ -178,6 +190,10 @@ __host__ __device__ inline void make_view_hdr(const Geom& g, float ang, ViewHdr&
     h.c = cos(h.beta);
     h.sx = -h.s * g.sod;
     h.sy = h.c * g.sod;
+    h.sf = (float)h.s;
+    h.cf = (float)h.c;
+    h.sxr = (float)h.sx;
+    h.syr = (float)h.sy;
     h.spar = h.use_x ? h.sx : h.sy;
     h.sperp = h.use_x ? h.sy : h.sx;
     h.nlines = h.use_x ? g.H : g.W;
@@ -381,6 +397,27 @@ __device__ __forceinline__ float guess_atan2f(float y, float x) {
     return y < 0.0f ? -r : r;
 }
 constexpr float XR_GUESS_ATAN_ERR = 4.0e-6f;  // bound used to widen brackets
+
+// The same with an eight-term polynomial fitted the same way (max error 1.2e-7
+// rad in FP32, its rounding), for callers that take the column as it is.
+__device__ __forceinline__ float fine_atan2f(float y, float x) {
+    const float ax = fabsf(x), ay = fabsf(y);
+    const float mx = fmaxf(ax, ay), mn = fminf(ax, ay);
+    const float t = mx > 0.0f ? mn * rcp_fast(mx) : 0.0f;
+    const float t2 = t * t;
+    float p = -0.0040545593947172165f;
+    p = fmaf(p, t2, 0.021862929686903954f);
+    p = fmaf(p, t2, -0.055912286043167114f);
+    p = fmaf(p, t2, 0.09642194211483002f);
+    p = fmaf(p, t2, -0.1390862911939621f);
+    p = fmaf(p, t2, 0.19946564733982086f);
+    p = fmaf(p, t2, -0.33329859375953674f);
+    p = fmaf(p, t2, 0.9999993443489075f);
+    float r = t * p;
+    if (ay > ax) r = 1.5707963267948966f - r;
+    if (x < 0.0f) r = 3.141592653589793f - r;
+    return y < 0.0f ? -r : r;
+}
 
 // Fractional traversal index of the detector position hit by the ray
 // source -> world point (x, y).  FP32 guess only; callers verify against the

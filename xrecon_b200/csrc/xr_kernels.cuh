@@ -116,47 +116,47 @@ __device__ __forceinline__ void setup_view_entry(const Geom& g, const int dim3d,
 
     const size_t oc = (size_t)v * g.Nu + k;
     const double Dk1 = arcf ? arc_boundary_f(g, h, k + 1, angle, ea, eb) : boundary_axis(g, h, (double)k + 1.0, uscale);
-    auto put_R = [&](double R) {
-        vt.colR[oc] = R;
+    const double dperp = h.use_x ? g.dy : g.dx;
+    // colQ = Q, colR = R, colE = E and the FP32 column steps (2D carries E in
+    // them, and has neither colQ nor colR)
+    auto put = [&](double Q, double R, float E) {
+        if (vt.colQ) vt.colQ[oc] = Q;
+        if (vt.colR) vt.colR[oc] = R;
+        vt.colE[oc] = E;
         if (vt.colWR) {
             double A1, B1;
             boundary_line_coeffs(g, h, Dk1, A1, B1);
-            const float hi = (float)R;
-            vt.colWR[oc] = make_float4((float)(A1 - A), (float)(B1 - B), hi, (float)(R - (double)hi));
+            const float hi = dim3d ? (float)R : E;
+            vt.colWR[oc] = make_float4((float)(A1 - A), (float)(B1 - B), hi, dim3d ? (float)(R - (double)hi) : 0.0f);
         }
     };
-    const double dperp = h.use_x ? g.dy : g.dx;
     if (g.type == GEO_PARALLEL) {
         // forward3d.cpp:58,98 (xy_scale / dv) and system_matrix2d.cpp:109.
-        vt.colQ[oc] = 1.0 / g.dz;
-        put_R(g.dz);
-        vt.colE[oc] = (float)(dim3d ? dperp / (g.du * g.dv) : dperp / g.du);
+        put(1.0 / g.dz, g.dz, (float)(dim3d ? dperp / (g.du * g.dv) : dperp / g.du));
         vt.colF[oc] = 1.0f;
         vt.colM[oc] = 0.0f;
         return;
     }
-    double M;
-    if (arcf) {
-        // column centre at the float32 centre angle (forward3d.cpp:285-297)
-        const double ac = (double)arc_angle_f(g, h.keep, (float)k + 0.5f, angle);
-        const double cx = sin(ac) * g.sdd + h.sx, cy = -cos(ac) * g.sdd + h.sy;
-        M = h.use_x ? h.sy / (h.sy - cy) : h.sx / (h.sx - cx);
-    } else {
-        M = column_mag(g, h, k, uscale);
-    }
-    vt.colQ[oc] = M / g.dz;
-    put_R(g.dz / M);
     const double aa = 0.5 * (Dk + Dk1) - h.spar;
     const double F = aa * aa + h.sperp * h.sperp;
+    double M = 1.0;
     if (dim3d) {
+        if (arcf) {
+            // column centre at the float32 centre angle (forward3d.cpp:285-297)
+            const double ac = (double)arc_angle_f(g, h.keep, (float)k + 0.5f, angle);
+            const double cx = sin(ac) * g.sdd + h.sx, cy = -cos(ac) * g.sdd + h.sy;
+            M = h.use_x ? h.sy / (h.sy - cy) : h.sx / (h.sx - cx);
+        } else {
+            M = column_mag(g, h, k, uscale);
+        }
         // s_A = dperp / (area * triangle_cosine): forward3d.cpp:331-343.
         const double rs = (g.type == GEO_FLAT) ? g.sod / g.sdd : 1.0;
-        vt.colE[oc] = (float)(dperp / (fabs(h.sperp) * (Dk1 - Dk) * M * g.dv * rs));
+        put(M / g.dz, g.dz / M, (float)(dperp / (fabs(h.sperp) * (Dk1 - Dk) * M * g.dv * rs)));
         vt.colF[oc] = (float)F;
         vt.colM[oc] = (float)M;
     } else {
         // 2D: dperp / ((D1 - D0) * cos_weight), system_matrix2d.cpp:213,251.
-        vt.colE[oc] = (float)(dperp * sqrt(F) / (fabs(h.sperp) * (Dk1 - Dk)));
+        put(M / g.dz, g.dz / M, (float)(dperp * sqrt(F) / (fabs(h.sperp) * (Dk1 - Dk))));
         vt.colF[oc] = 1.0f;
         vt.colM[oc] = 0.0f;
     }
@@ -274,7 +274,7 @@ cell_gather3d_kernel(const Geom g, const ViewTables vt, const TI* __restrict__ v
     const size_t plane = (size_t)nlines * npix;
     const TI* __restrict__ vol = (h.use_x ? vol_rows : vol_cols) + (size_t)b * g.D * plane;
     const double zr0 = zd0 + r0 * dvv;
-    // arc detector, B^T / Bw^T: chained column walks (see cell2d_sum)
+    // arc detector, B^T / Bw^T: chained column walks (see cell2d_walk)
     const bool chain = (MODE == OP_BT || MODE == OP_BWT) && !HEL && vt.arc;
     const float4* __restrict__ ea = chain ? vt.arc + 2 * (size_t)v * (Nu + 1) : nullptr;
     float d1 = 0.0f;
@@ -599,240 +599,6 @@ vox_gather3d_kernel(const Geom g, const GeomF gf, const ViewTables vt, const TI*
         const int j = j0 + i;
         if (j < g.D) st(vol + (((size_t)b * g.D + j) * g.H + iy) * g.W + ix, acc[i]);
     }
-}
-
-// ------------------------------------------------------------- 2D kernels
-
-// Cell gather, 2D: one thread per (view, column).
-template <typename TI, int MODE>
-__device__ __forceinline__ float cell2d_sum(const Geom& g, const ViewTables& vt, const ViewHdr& h,
-                                            const TI* __restrict__ img_rows, const TI* __restrict__ img_cols,
-                                            const int v, const int k, const float cw, const int l0, const int ls);
-template <typename TI, int MODE>
-__device__ __forceinline__ float pix2d_sum(const Geom& g, const ViewTables& vt, const TI* __restrict__ sinob,
-                                           const int ix, const int iy, const float cw, const int v0,
-                                           const int v1, const int vs);
-
-template <typename TI, typename TO, int MODE>
-__global__ void __launch_bounds__(128)
-cell_gather2d_kernel(const Geom g, const ViewTables vt, const TI* __restrict__ img_rows,
-                     const TI* __restrict__ img_cols, TO* __restrict__ sino, const int nview,
-                     const float cw) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int v = blockIdx.y, b = blockIdx.z;
-    const int Nu = g.Nu;
-    if (k >= Nu) return;
-    const ViewHdr h = vt.hdr[v];
-    const size_t plane = (size_t)g.W * g.H;
-    const float acc = cell2d_sum<TI, MODE>(g, vt, h, img_rows + b * plane, img_cols + b * plane, v, k, cw, 0, 1);
-    const int col = h.keep ? k : Nu - 1 - k;
-    st(sino + ((size_t)b * nview + v) * Nu + col, acc);
-}
-
-// Cell k of view v (traversal order), lines L = l0, l0 + ls, ...: the 2D DD
-// line sum, times the cell scale colE for MODE OP_A (applied by the caller
-// when the lines are split over threads: pass ls > 1 and scale afterwards).
-template <typename TI, int MODE>
-__device__ __forceinline__ float cell2d_sum(const Geom& g, const ViewTables& vt, const ViewHdr& h,
-                                            const TI* __restrict__ img_rows, const TI* __restrict__ img_cols,
-                                            const int v, const int k, const float cw, const int l0, const int ls) {
-    const int Nu = g.Nu;
-    const size_t ob = (size_t)v * (Nu + 1) + k;
-    const double bA0 = vt.bA[ob], bB0 = vt.bB[ob], bA1 = vt.bA[ob + 1], bB1 = vt.bB[ob + 1];
-    const int nlines = h.nlines, npix = h.npix;
-    const TI* __restrict__ img = h.use_x ? img_rows : img_cols;
-    const float dpixf = (float)h.dpix;
-    // arc detector, B^T / Bw^T: the column's upper boundary on the chained
-    // walk of a pixel whose first edge lies in this column (every pixel but
-    // the band's first); the same on every line
-    const bool chain = (MODE == OP_BT || MODE == OP_BWT) && vt.arc;
-    const float4* __restrict__ ea = chain ? vt.arc + 2 * (size_t)v * (Nu + 1) : nullptr;
-    float d1 = 0.0f;
-    if (chain) {
-        ArcChain ch;
-        ch.start(ea, k, h.keep, (float)g.du);
-        d1 = ch.next_exact(h, ea, k + 1);
-        if (k + 1 == Nu) d1 = fminf(d1, 0.0f);
-    }
-    float acc = 0.0f;
-    for (int L = l0; L < nlines; L += ls) {
-        const double pk = fma(bB0, (double)L, bA0);
-        const double pk1 = fma(bB1, (double)L, bA1);
-        const int pa = max((int)floor(pk), 0);
-        const int pb = min((int)ceil(pk1) - 1, npix - 1);
-        if (pa > pb) continue;
-        float lf;
-        if (MODE == OP_A) lf = __fdividef(dpixf, (float)fma(h.q1, (double)L, h.q0));
-        else lf = cw;
-        const TI* __restrict__ line = img + (size_t)L * npix;
-        // boundaries relative to the first pixel, so FP32 keeps them exact
-        float u0 = (float)(pk - (double)pa), u1 = (float)(pk1 - (double)pa);
-        float u1b = u1;  // upper boundary for the band's later pixels
-        if (chain) {
-            const float qd = (float)(fma(h.q1, (double)L, h.q0) / h.dpix);
-            u1b = fmaf(d1, qd, u1);
-            u1 = u1b;
-            if (k > 0 && pk > (double)pa)
-                arc_first_pixel_bounds(g, vt, h, ea, v, k, L, pa, pk, pk1, qd, u0, u1);
-        }
-        for (int pp = pa; pp <= pb; ++pp) {
-            const float o = (float)(pp - pa);
-            float w = (fminf(o + 1.0f, pp == pa ? u1 : u1b) - fmaxf(o, u0)) * lf;
-            if (MODE == OP_BWT) {
-                float px, py;
-                pixel_center(g, h, L, pp, px, py);
-                w *= fbp_weight(g, h, px, py);
-            }
-            acc = fmaf(w, ld(line + XR_BOUND(pp, 0, npix - 1)), acc);
-        }
-    }
-    if (MODE == OP_A && ls == 1) acc *= vt.colE[(size_t)v * Nu + k];
-    return acc;
-}
-
-// Voxel gather, 2D: one thread per pixel, sweeping the views.
-template <typename TI, typename TO, int MODE>
-__global__ void __launch_bounds__(256)
-vox_gather2d_kernel(const Geom g, const ViewTables vt, const TI* __restrict__ sino, TO* __restrict__ img,
-                    const int nview, const float cw, const float oscale) {
-    const int ix = blockIdx.x * blockDim.x + threadIdx.x;
-    const int iy = blockIdx.y * blockDim.y + threadIdx.y;
-    const int b = blockIdx.z;
-    if (ix >= g.W || iy >= g.H) return;
-    const float acc = pix2d_sum<TI, MODE>(g, vt, sino + (size_t)b * nview * g.Nu, ix, iy, cw, 0, nview, 1);
-    st(img + ((size_t)b * g.H + iy) * g.W + ix, acc * oscale);
-}
-
-// Pixel (ix, iy): the 2D DD backprojection sum over views v = v0, v0 + vs, ...
-// < v1 of the sinogram sinob [nview][Nu].
-template <typename TI, int MODE>
-__device__ __forceinline__ float pix2d_sum(const Geom& g, const ViewTables& vt, const TI* __restrict__ sinob,
-                                           const int ix, const int iy, const float cw, const int v0,
-                                           const int v1, const int vs) {
-    const int Nu = g.Nu;
-    // This pixel's edges and centre in world coordinates (the values
-    // line_point and pixel_center give), hoisted out of the view loop.
-    const float dxf = (float)g.dx, dyf = (float)g.dy;
-    const float xa_x = (float)(-0.5 * g.W * g.dx + g.shx) + (float)ix * dxf;   // x-axis views: x edges
-    const float yc_x = (float)((0.5 * g.H - iy - 0.5) * g.dy + g.shy);          //   and line centre
-    const float xc_y = (float)((ix - 0.5 * g.W + 0.5) * g.dx + g.shx);          // y-axis views: line centre
-    const float ya_y = (float)(-0.5 * g.H * g.dy + g.shy) + (float)(g.H - 1 - iy) * dyf;  //   and y edges
-    const float pcx = (float)((ix - 0.5 * g.W + 0.5) * g.dx + g.shx);  // pixel centre
-    const float pcy = (float)((0.5 * g.H - iy - 0.5) * g.dy + g.shy);
-    const float sodf = (float)g.sod, shuf = (float)g.shu, inv_du = (float)(1.0 / g.du);
-    const float inv_dx = (float)(1.0 / g.dx), inv_dy = (float)(1.0 / g.dy);
-    // column bracket margin: half a column, plus the arc guess's angle error
-    const float margin = 0.5f + (g.type == GEO_ARC ? XR_GUESS_ATAN_ERR * inv_du : 0.0f);
-    float acc = 0.0f;
-    for (int v = v0; v < v1; v += vs) {
-        const ViewHdr& h = vt.hdr[v];
-        int L, p;
-        float xa, ya, xb, yb;
-        if (h.use_x) {
-            L = iy; p = ix;
-            xa = xa_x; xb = xa_x + dxf; ya = yb = yc_x;
-        } else {
-            L = ix; p = g.H - 1 - iy;
-            xa = xb = xc_y; ya = ya_y; yb = ya_y + dyf;
-        }
-        float lf;
-        if (MODE == OP_AT) {
-            lf = __fdividef((float)h.dpix, (float)fma(h.q1, (double)L, h.q0));
-        } else {
-            lf = cw;
-            if (MODE == OP_BW) lf *= fbp_weight(g, h, pcx, pcy);
-        }
-        // FP32 column guess (brackets the overlapped columns; the overlaps
-        // themselves come from the FP64 boundary tables)
-        const float sf = (float)h.s, cf = (float)h.c;
-        float kf0, kf1;
-        if (g.type == GEO_FLAT) {
-            kf0 = (__fdividef(sodf * (xa * cf + ya * sf), sodf + xa * sf - ya * cf) - shuf) * inv_du;
-            kf1 = (__fdividef(sodf * (xb * cf + yb * sf), sodf + xb * sf - yb * cf) - shuf) * inv_du;
-        } else if (g.type == GEO_ARC) {
-            // One guess, at the pixel centre, and a bound on the footprint's
-            // half-width: the segment between the pixel's edges on this line
-            // (half-length a) seen from the source at distance r from its
-            // centre spans at most asin(a / r) <= a / (r - a) rad on each
-            // side.  The bracket may take a column more than the edges'
-            // own guesses would; the walk skips it.
-            const float dcx = h.dcx, dcy = h.dcy;
-            const float ex = pcx - (float)h.sx, ey = pcy - (float)h.sy;
-            const float kc = guess_atan2f(dcx * ey - dcy * ex, dcx * ex + dcy * ey) * inv_du;
-            const float a = 0.5f * (h.use_x ? dxf : dyf);
-            const float r2 = fmaf(ex, ex, ey * ey);
-            const float r = r2 * rsqrtf(r2);
-            const float hw = __fdividef(a, fmaxf(r - a, a)) * inv_du * 1.001f;
-            kf0 = kc - hw;
-            kf1 = kc + hw;
-        } else {
-            kf0 = (xa * cf + ya * sf - shuf) * inv_du;
-            kf1 = (xb * cf + yb * sf - shuf) * inv_du;
-        }
-        if (h.keep) { kf0 += 0.5f * Nu; kf1 += 0.5f * Nu; }
-        else { kf0 = 0.5f * Nu - kf0; kf1 = 0.5f * Nu - kf1; }
-        const float lo = fmaxf(fminf(fminf(kf0, kf1), (float)Nu + 2.0f), -2.0f);
-        const float hi = fmaxf(fminf(fmaxf(kf0, kf1), (float)Nu + 2.0f), -2.0f);
-        const int ka = max(0, (int)floorf(lo - margin));
-        const int kb = min(Nu - 1, (int)floorf(hi + margin));
-        if (ka > kb) continue;
-        const double* __restrict__ bA = vt.bA + (size_t)v * (Nu + 1);
-        const double* __restrict__ bB = vt.bB + (size_t)v * (Nu + 1);
-        const TI* __restrict__ sv = sinob + (size_t)v * Nu;
-        const double dp = (double)p, dL = (double)L;
-        if (MODE != OP_AT && vt.arc) {
-            // arc detector: the pixel's columns walked with chained angles.
-            // Boundary ka relative to the pixel in FP64, the next direct
-            // boundaries (pd) by adding the columns' widths on this line in
-            // FP32, which the walk's arc entries carry.
-            const float4* __restrict__ ea = vt.arc + 2 * (size_t)v * (Nu + 1);
-            const float Lf = (float)L;
-            const float qd = (float)fma(h.q1, dL, h.q0) * (h.use_x ? inv_dx : inv_dy);  // pixels per axis unit
-            auto width = [&](int j) { const float4 a = ea[2 * j]; return fmaf(a.w, Lf, a.z); };
-            int k = ka;
-            float pkl = (float)(fma(bB[k], dL, bA[k]) - dp);
-            float pd = pkl + width(k + 1);
-            while (!(pd > 0.0f) && k < kb) {
-                ++k;
-                pkl = pd;
-                pd += width(k + 1);
-            }
-            ArcChain ch;
-            ch.start(ea, k, h.keep, (float)g.du);
-            float d = ch.next_linear(ea, k + 1);
-            if (k + 1 == Nu) d = fminf(d, 0.0f);  // the detector's end
-            float pk1 = fmaf(d, qd, pd);
-            for (;;) {
-                const float wd = fminf(1.0f, pk1) - fmaxf(0.0f, pkl);
-                if (wd > 0.0f) {
-                    const int col = h.keep ? k : Nu - 1 - k;
-                    acc = fmaf(wd * lf, ld(sv + XR_BOUND(col, 0, Nu - 1)), acc);
-                }
-                if (++k > kb) break;
-                pkl = pk1;
-                if (pkl >= 1.0f) break;
-                float w;
-                d = ch.next_linear(ea, k + 1, Lf, w);
-                if (k + 1 == Nu) d = fminf(d, 0.0f);
-                pd += w;
-                pk1 = fmaf(d, qd, pd);
-            }
-            continue;
-        }
-        // boundaries relative to the pixel (pixel units)
-        float pkl = (float)(fma(bB[ka], dL, bA[ka]) - dp);
-        for (int k = ka; k <= kb; ++k) {
-            const float pk1 = (float)(fma(bB[k + 1], dL, bA[k + 1]) - dp);
-            const float wd = fminf(1.0f, pk1) - fmaxf(0.0f, pkl);
-            pkl = pk1;
-            if (!(wd > 0.0f)) continue;
-            float w = wd * lf;
-            if (MODE == OP_AT) w *= vt.colE[(size_t)v * Nu + k];
-            const int col = h.keep ? k : Nu - 1 - k;
-            acc = fmaf(w, ld(sv + XR_BOUND(col, 0, Nu - 1)), acc);
-        }
-    }
-    return acc;
 }
 
 // -------------------------------------------------------------- FBP filter

@@ -13,15 +13,16 @@
 //      256 / CW threads of a column split its lines and reduce in shared
 //      memory;
 //   2  FBP pre-filter of every sinogram row: cosine weight x correlation with
-//      the instance's filter taps (the same arithmetic as fbp_filter_kernel);
+//      the instance's filter taps (the same arithmetic as fbp_filter_kernel),
+//      then the filtered row's table for the next phase (xr_dd2d.cuh);
 //   3  weighted backprojection Bw of the filtered rows times the FBP scale,
-//      pixel-owned: a tile is 256 / VS pixels, the VS threads of a pixel
-//      split its views and reduce in shared memory.
+//      pixel-owned: a tile is 8 / VS warps of 2 x 2 pixel blocks (xr_dd2d.cuh),
+//      VS warps split a block's views and reduce in shared memory.
 // CW and VS are launch parameters chosen by the autotuner of the Python
 // wrapper.  No atomics touch data: the counters only hand out tiles.
 #pragma once
 
-#include "xr_kernels.cuh"
+#include "xr_dd2d.cuh"
 #include "xr_tma.cuh"
 
 namespace xr {
@@ -34,6 +35,7 @@ __device__ long long g_barrier_limit = XR_BARRIER_LIMIT_DEFAULT;
 // One instance, device side (pointers already resolved).
 struct RaggedDev {
     Geom g;
+    Geom2F f;
     ViewTables vt;
     int nview;
     float cw;       // backprojection column width
@@ -42,6 +44,8 @@ struct RaggedDev {
     float* imgT;
     float* sino;
     float* filt_out;
+    RowTable tab;   // row tables of filt_out and their flags (xr_dd2d.cuh)
+    int* flags;
     float* recon;
     const float* ang;
     const float* filt;
@@ -107,10 +111,21 @@ __device__ __forceinline__ int next_tile(int* ctr) {
     return t_s;
 }
 
+// Filtered rows of one view; written by this kernel, so not through __ldg.
+struct FiltLanes {
+    const float* p;
+    __device__ __forceinline__ Lanes<1> operator()(int col) const {
+        Lanes<1> r;
+        r.v[0] = p[col];
+        return r;
+    }
+};
+
 __global__ void __launch_bounds__(256, 3)
 ragged2d_fbp_kernel(const RaggedDev* __restrict__ inst, const int ninst, const int4 totals, const int4 lists,
                     const int project, const int CW, const int VS, unsigned* bar, int* ctr) {
     extern __shared__ float sm[];
+    __shared__ double2 row_sums[8];
     const int tid = threadIdx.x;
     const unsigned nb = gridDim.x;
 
@@ -145,15 +160,19 @@ ragged2d_fbp_kernel(const RaggedDev* __restrict__ inst, const int ninst, const i
             const int v = lt / nbk, kb = lt - v * nbk;
             const int c = tid % CW, s = tid / CW;
             const int k = kb * CW + c;
-            const ViewHdr h = I.vt.hdr[v];
+            const ViewHdr& h = I.vt.hdr[v];
+            const float* img = h.use_x ? I.img : I.imgT;
+            const int npix = h.npix;
             float acc = 0.0f;
-            if (k < g.Nu) acc = cell2d_sum<float, OP_A>(g, I.vt, h, I.img, I.imgT, v, k, 0.0f, s, LS);
+            if (k < g.Nu)
+                cell2d_walk<OP_A>(g, I.f, I.vt, h, v, k, 0.0f, s, LS,
+                                  [&](int L, int p, float w) { acc = fmaf(w, img[L * npix + p], acc); });
             sm[tid] = acc;
             __syncthreads();
             if (s == 0 && k < g.Nu) {
                 float sum = 0.0f;
                 for (int j = 0; j < LS; ++j) sum += sm[j * CW + c];
-                if (LS > 1) sum *= I.vt.colE[(size_t)v * g.Nu + k];  // LS == 1: applied by cell2d_sum
+                sum *= I.vt.colE[(size_t)v * g.Nu + k];
                 const int col = h.keep ? k : g.Nu - 1 - k;
                 I.sino[(size_t)v * g.Nu + col] = sum;
             }
@@ -183,28 +202,48 @@ ragged2d_fbp_kernel(const RaggedDev* __restrict__ inst, const int ninst, const i
             if (j < Nu) a0 = fmaf(x[j], fi[j], a0);
             I.filt_out[(size_t)v * Nu + i] = a0 + a1;
         }
+        __syncthreads();  // the whole row is in filt_out
+        const float* y = I.filt_out + (size_t)v * Nu;
+        const int keep = I.vt.hdr[v].keep;
+        const bool bad = build_row_table(I.vt, v, Nu, I.tab.at(v, Nu), row_sums,
+                                         [&](int j) -> float { return y[keep ? j : Nu - 1 - j]; });
+        if (tid == 0) I.flags[v] = bad;
     }
     if (!grid_barrier(bar, nb)) return;
 
     // phase 3: weighted backprojection x FBP scale
     {
-        const int PX = blockDim.x / VS;
+        const int ntile = 8 / VS, lane = tid & 31, wp = tid >> 5, slice = wp / ntile;
         for (int t = next_tile(&ctr[3]); t < totals.w; t = next_tile(&ctr[3])) {
             const RaggedDev& I = inst[find_instance(inst, ninst, lists.w, t)];
-            const Geom& g = I.g;
-            const int p = tid % PX, s = tid / PX;
-            const int idx = (t - I.t0[lists.w]) * PX + p;
-            float acc = 0.0f;
-            if (idx < g.H * g.W) {
-                const int iy = idx / g.W, ix = idx - iy * g.W;
-                acc = pix2d_sum<float, OP_BW>(g, I.vt, I.filt_out, ix, iy, I.cw, s, I.nview, VS);
-            }
-            sm[tid] = acc;
+            const int W = I.f.W, H = I.f.H;
+            int ix0, iy0;
+            pix2t_origin(I.f, VS, t - I.t0[lists.w], wp % ntile, lane, ix0, iy0);
+            const bool active = ix0 < W && iy0 < H;
+            float acc[P2][P2] = {};
+            if (active)
+                for (int v = slice; v < I.nview; v += VS) {
+                    if (I.flags[v]) {
+                        const float4 s = pix2d_view_walk<OP_BW>(I.f, I.vt, v, ix0, iy0, I.cw,
+                                                                FiltLanes{I.filt_out + (size_t)v * I.f.Nu});
+                        acc[0][0] += s.x; acc[0][1] += s.y; acc[1][0] += s.z; acc[1][1] += s.w;
+                    } else {
+                        pix2t_view<OP_BW>(I.f, I.vt, v, ix0, iy0, I.cw, I.tab.at(v, I.f.Nu), acc);
+                    }
+                }
+            float* a = &acc[0][0];
+#pragma unroll
+            for (int e = 0; e < P2 * P2; ++e) sm[e * 256 + tid] = a[e];
             __syncthreads();
-            if (s == 0 && idx < g.H * g.W) {
-                float sum = 0.0f;
-                for (int j = 0; j < VS; ++j) sum += sm[j * PX + p];
-                I.recon[idx] = sum * I.scale;
+            if (!slice && active) {
+                for (int s = 1; s < VS; ++s)
+#pragma unroll
+                    for (int e = 0; e < P2 * P2; ++e) a[e] += sm[e * 256 + s * ntile * 32 + tid];
+#pragma unroll
+                for (int r = 0; r < P2; ++r)
+#pragma unroll
+                    for (int c = 0; c < P2; ++c)
+                        if (ix0 + c < W && iy0 + r < H) I.recon[(iy0 + r) * W + ix0 + c] = acc[r][c] * I.scale;
             }
         }
     }
