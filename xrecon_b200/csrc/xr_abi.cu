@@ -157,10 +157,19 @@ bool arc_chain_op(const Geom& g, int op) {
 
 // ------------------------------------------------------ TMA staging plans
 
+// Window plan of the projection for one launch shape: NW warps of R rows each.
 struct CellPlan {
     bool ok;
-    int BP, BZ, R;
+    int BP, BZ, R, NW;
     bool fine;  // rows longer than a voxel are rare: the fine-only kernel
+    int NB;     // pixels of a column per pass of the walk
+};
+
+// The plan of the default shape (eight warps of 8 or 16 rows), which decides
+// whether the staged projection is taken at all, and the one it is launched
+// with.
+struct CellPlans {
+    CellPlan base, launch;
 };
 
 constexpr int CELL_NW = 8;
@@ -169,37 +178,63 @@ int cell_rows_per_thread(const Geom& g) { return g.Nv >= 128 ? 16 : 8; }
 
 int round_up(int v, int m) { return (v + m - 1) / m * m; }
 
+// Launch shape for Nv detector rows: a warp's time per line is its R rows plus
+// a line setup worth about nine of them, so longer runs of rows pay the setup
+// less often, while rows past the detector are walked for nothing and a CTA
+// of one warp waits on its own copies (us for R = 16 / 32: 64 rows 4512 / 3758,
+// 83 rows 1281 / 1083, 96 rows 6643 / 5140, 160 rows 5266 / 4971; 32 rows, one
+// warp at R = 32, 877 / 1734; eight warps of 8 or 16 rows took 5858, 1895, 9143,
+// 6888 and 1748).
+void cell_shape(int Nv, bool fine, int& R, int& NW) {
+    int best = 1 << 30;
+    for (int r = fine ? 8 : 16; r <= (fine ? 32 : 16); r *= 2) {
+        // rows of a CTA: at most 128, split evenly over the fewest CTAs
+        const int groups = (Nv + 127) / 128, per = (Nv + groups - 1) / groups, nw = (per + r - 1) / r;
+        if (nw > CELL_NW || (fine && nw == 1 && r > 8)) continue;
+        const int cost = groups * nw * (r + 9);
+        if (cost <= best) best = cost, R = r, NW = nw;
+    }
+}
+
+size_t cell_smem(const CellPlan& p, int maxlines) {
+    return (size_t)CELL_NS * cell_stage_elems<float>(p.BP, p.BZ) * 4 + 8 * CELL_NS + (size_t)maxlines * 16;
+}
+
 // Sizes the line window of the TMA cell gather for this geometry by
 // evaluating the kernel's own window function over the CTAs of views sampled
 // densely in angle (the window depends on the angle only through smooth
 // functions; the 45-degree axis switches are sampled on both sides).  Cached
 // per geometry.
-CellPlan plan_cell(const Geom& g) {
+CellPlans plan_cell_shapes(const Geom& g, int cap_z) {
     static std::mutex mu;
-    static std::map<std::string, CellPlan> cache;
-    const std::string key(reinterpret_cast<const char*>(&g), sizeof(Geom));
+    static std::map<std::string, CellPlans> cache;
+    std::string key(reinterpret_cast<const char*>(&g), sizeof(Geom));
+    key.append(reinterpret_cast<const char*>(&cap_z), sizeof(int));
     {
         std::lock_guard<std::mutex> lk(mu);
         auto it = cache.find(key);
         if (it != cache.end()) return it->second;
     }
-    CellPlan p{false, 0, 0, cell_rows_per_thread(g), false};
-    double coarse = 0.0, pairs = 0.0;
-    const int RG = CELL_NW * p.R;
+    double coarse = 0.0, wide = 0.0, pairs = 0.0;
     const double uscale = (g.type == GEO_FLAT) ? g.sod / g.sdd : 1.0;
     const double rs = (g.type == GEO_FLAT) ? g.sod / g.sdd : 1.0;
     const double zd0 = (-0.5 * g.Nv * g.dv + g.shv) * rs, dvv = g.dv * rs;
     const double z0dz = (-0.5 * g.D * g.dz + g.shz) / g.dz;
+    // rows per CTA: the default shape's, and that of every shape the launch may take
+    CellPlan def{false, 0, 0, cell_rows_per_thread(g), CELL_NW, false, 2};
+    int shapes[3][2] = {{def.R, def.NW}, {0, 0}, {0, 0}};
+    cell_shape(g.Nv, false, shapes[1][0], shapes[1][1]);
+    cell_shape(g.Nv, true, shapes[2][0], shapes[2][1]);
+    int maxspan = 0;
+    double maxnz[3] = {0.0, 0.0, 0.0};
     std::vector<double> A(g.Nu + 1), B(g.Nu + 1), Q(g.Nu);
     std::vector<double> angles;
-    const int NS = 256;
-    for (int i = 0; i < NS; ++i) angles.push_back(2.0 * M_PI * i / NS + 0.37 / NS);
+    const int NSA = 256;
+    for (int i = 0; i < NSA; ++i) angles.push_back(2.0 * M_PI * i / NSA + 0.37 / NSA);
     for (int i = 0; i < 8; ++i) {
         angles.push_back(M_PI / 4 * i + 1e-5);
         angles.push_back(M_PI / 4 * i - 1e-5);
     }
-    int maxspan = 0;
-    double maxnz = 0.0;
     for (double ang : angles) {
         ViewHdr h;
         make_view_hdr(g, (float)ang, h);
@@ -215,11 +250,15 @@ CellPlan plan_cell(const Geom& g) {
             for (int k = 0; k < g.Nu; ++k) {
                 const double a0 = std::fabs(Q[k] * dvv * h.q0);
                 const double a1 = std::fabs(Q[k] * dvv * (h.q0 + h.q1 * (n - 1.0)));
-                double f;
-                if (a0 >= 0.999 && a1 >= 0.999) f = 1.0;
-                else if (a0 < 0.999 && a1 < 0.999) f = 0.0;
-                else f = (std::max(a0, a1) - 0.999) / std::fabs(a1 - a0);
-                coarse += f;
+                // share of the lines on which an affine term exceeds `lim`
+                auto above = [](double x0, double x1, double lim) {
+                    if (x0 >= lim && x1 >= lim) return 1.0;
+                    if (x0 < lim && x1 < lim) return 0.0;
+                    return (std::max(x0, x1) - lim) / std::fabs(x1 - x0);
+                };
+                coarse += above(a0, a1, 0.999);
+                const double dA = A[k + 1] - A[k], dB = B[k + 1] - B[k];
+                wide += above(std::fabs(dA), std::fabs(dA + dB * (n - 1.0)), 1.03);
                 pairs += 1.0;
             }
         }
@@ -229,29 +268,51 @@ CellPlan plan_cell(const Geom& g) {
             c.bAk0 = A[k0]; c.bBk0 = B[k0]; c.bAke = A[kend]; c.bBke = B[kend];
             c.Qmin = 1e300; c.Qmax = -1e300;
             for (int k = k0; k < kend; ++k) { c.Qmin = std::min(c.Qmin, Q[k]); c.Qmax = std::max(c.Qmax, Q[k]); }
-            for (int rg0 = 0; rg0 < g.Nv; rg0 += RG) {
-                c.zlo = zd0 + rg0 * dvv;
-                c.zhi = zd0 + (rg0 + RG) * dvv;
-                for (int L : {0, h.nlines - 1}) {
-                    const CellWindow w = cell_window(c, h, L, z0dz, h.npix, g.D, 1 << 30, 1 << 30);
-                    if (w.empty) continue;
-                    const double ph = std::fma(c.bBke, (double)L, c.bAke);
-                    const int phi = std::min((int)std::ceil(ph) - 1, h.npix - 1);
-                    maxspan = std::max(maxspan, phi - w.p0 + 1);
-                    maxnz = std::max(maxnz, (double)(w.zlast - w.z0 + 1));
+            for (int sh = 0; sh < 3; ++sh) {
+                const int RG = shapes[sh][0] * shapes[sh][1];
+                for (int rg0 = 0; rg0 < g.Nv; rg0 += RG) {
+                    c.zlo = zd0 + rg0 * dvv;
+                    c.zhi = zd0 + (rg0 + RG) * dvv;
+                    for (int L : {0, h.nlines - 1}) {
+                        const CellWindow w = cell_window(c, h, L, z0dz, h.npix, g.D, 1 << 30, 1 << 30);
+                        if (w.empty) continue;
+                        const double ph = std::fma(c.bBke, (double)L, c.bAke);
+                        const int phi = std::min((int)std::ceil(ph) - 1, h.npix - 1);
+                        maxspan = std::max(maxspan, phi - w.p0 + 1);
+                        maxnz[sh] = std::max(maxnz[sh], (double)(w.zlast - w.z0 + 1));
+                    }
                 }
             }
         }
     }
-    p.fine = pairs > 0.0 && coarse < 0.05 * pairs;
-    p.BP = round_up(std::max(maxspan, 8), 8);
-    p.BZ = (int)maxnz;
-    p.ok = p.BP <= 256 && p.BZ <= 256 && p.BZ >= 1 &&
-           (size_t)CELL_NS * p.BP * (p.BZ + 1) * 4 + (size_t)std::max(g.W, g.H) * 16 + 8 * CELL_NS <= 200 * 1024;
+    const bool fine = pairs > 0.0 && coarse < 0.05 * pairs;
+    // a column of width w pixels overlaps three with probability w - 1: above
+    // 1.03 some lane of most warps does, and the walk of two pixels a pass
+    // runs twice (us for 2 / 3 pixels a pass: 12 % of the lines 5829 / 6385,
+    // 22 % 5140 / 5245, 64 % 1033 / 877, 82 % 1463 / 1083)
+    const int nb = wide > 0.3 * pairs ? 3 : 2;
+    auto make = [&](int sh) {
+        CellPlan p{false, round_up(std::max(maxspan, 8), 8), std::min((int)maxnz[sh], cap_z), shapes[sh][0], shapes[sh][1], fine, nb};
+        p.ok = p.BP <= 256 && p.BZ <= 256 && p.BZ >= 1 &&
+               (size_t)CELL_NS * p.BP * (p.BZ + 1) * 4 + (size_t)std::max(g.W, g.H) * 16 + 8 * CELL_NS <= 200 * 1024;
+        return p;
+    };
+    CellPlans r;
+    r.base = make(0);
+    r.launch = make(fine ? 2 : 1);
+    // the default shape where the other's windows leave an SM fewer warps (its
+    // registers allow 16)
+    auto warps = [&](const CellPlan& p) {
+        const int per = (int)((228 * 1024) / (cell_smem(p, std::max(g.W, g.H)) + 1024));
+        return std::min(16, per * p.NW);
+    };
+    if (!r.launch.ok || warps(r.launch) < std::min(12, warps(r.base))) r.launch = r.base;
     std::lock_guard<std::mutex> lk(mu);
-    cache[key] = p;
-    return p;
+    cache[key] = r;
+    return r;
 }
+
+CellPlan plan_cell(const Geom& g) { return plan_cell_shapes(g, 1 << 30).base; }
 
 using EncodeTiledFn = PFN_cuTensorMapEncodeTiled_v12000;
 
@@ -602,11 +663,6 @@ constexpr int VOX_R = 16;
 constexpr int VOX_NW = 4;
 constexpr int PFX_NWY = XR_PFX_NWY;  // image lines (warps) per CTA
 
-template <typename T> constexpr int dtype_code();
-template <> constexpr int dtype_code<float>() { return DT_F32; }
-template <> constexpr int dtype_code<__nv_bfloat16>() { return DT_BF16; }
-template <> constexpr int dtype_code<__half>() { return DT_F16; }
-
 // Staged prefix gather (vox_stage3d_kernel), then its fallback launch for
 // the views a CTA could not stage; -1 when this geometry is not covered (the
 // caller then uses vox_prefix3d_kernel).
@@ -654,25 +710,25 @@ int run_pfx_stage(int eff, const Geom& g, const GeomF& gf, const ViewTables& vt,
                                                  z0dz, zd0, dvv, cw, atconst, oscale);
 }
 
-template <typename TI, typename TO, int R, int MODE, bool HEL>
+template <typename TO, int R, int MODE, bool HEL>
 int launch_cell_tma_mode(const Geom& g, const CellPlan& p, const CUtensorMap& mr, const CUtensorMap& mc,
-                         const TI* rows, const TI* cols, int pitch_r, int pitch_c, TO* out, int nbatch, int nview,
-                         const ViewTables& vt, cudaStream_t st, double z0dz, double zd0, double dvv, float cw,
+                         const float* rows, const float* cols, int pitch_r, int pitch_c, TO* out, int nbatch,
+                         int nview, const ViewTables& vt, cudaStream_t st, double z0dz, double zd0, double dvv, float cw,
                          const float* zwt) {
-    auto kern = p.fine ? cell_tma3d_kernel<TI, TO, R, 2, MODE, true, HEL>
-                       : cell_tma3d_kernel<TI, TO, R, 2, MODE, false, HEL>;
-    const int maxlines = std::max(g.W, g.H);
-    const size_t smem = CELL_NS * (size_t)cell_stage_elems<TI>(p.BP, p.BZ) * sizeof(TI) + 8 * CELL_NS +
-                        (size_t)maxlines * sizeof(int4);
+    auto kern = cell_tma3d_kernel<float, TO, R, 2, MODE, true, HEL>;
+    if (p.fine && p.NB == 3) kern = cell_tma3d_kernel<float, TO, R, 3, MODE, true, HEL>;
+    if constexpr (R <= 16)
+        if (!p.fine) kern = cell_tma3d_kernel<float, TO, R, 2, MODE, false, HEL>;
+    const size_t smem = cell_smem(p, std::max(g.W, g.H));
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return fail(XR_ERR_CUDA, "cannot reserve %zu bytes of shared memory", smem);
-    const int RG = CELL_NW * R;
+    const int RG = p.NW * R;
     const int total = nview * nbatch;
     for (int z0 = 0; z0 < total; z0 += 65535) {
         const int nz = std::min(65535, total - z0);
         dim3 grid((g.Nu + 31) / 32, (g.Nv + RG - 1) / RG, nz);
-        kern<<<grid, dim3(32, CELL_NW), smem, st>>>(g, vt, mr, mc, rows, cols, pitch_r, pitch_c, out, nview, z0, z0dz,
-                                                    zd0, dvv, cw, p.BP, p.BZ, zwt);
+        kern<<<grid, dim3(32, p.NW), smem, st>>>(g, vt, mr, mc, rows, cols, pitch_r, pitch_c, out, nview, z0, z0dz,
+                                                 zd0, dvv, cw, p.BP, p.BZ, zwt);
         if (int rc = check_cuda("cell_tma3d")) return rc;
     }
     return XR_OK;
@@ -683,26 +739,22 @@ int launch_cell_tma_mode(const Geom& g, const CellPlan& p, const CUtensorMap& mr
 // Window plan of a helical scan: the views' z placement varies, so the z
 // extent is sized on a volume deep enough that no window is clamped, then
 // capped at the real depth (a window never spans more than D + 2 slices).
-CellPlan plan_cell_helical(const Geom& g) {
+CellPlans plan_cell_helical(const Geom& g) {
     Geom gp = g;
     gp.D = 1 << 20;
     gp.shz = 0.0;
-    CellPlan p = plan_cell(gp);
-    p.BZ = std::min(p.BZ, g.D + 2);
-    p.ok = p.ok && p.BZ >= 1;
-    return p;
+    return plan_cell_shapes(gp, g.D + 2);
 }
 
-template <typename TI, typename TO, bool HEL = false>
-int run_cell_tma(int eff, const Geom& g, const TI* in, TO* out, int nbatch, int nview, char* ws, const Layout& l,
-                 const ViewTables& vt, cudaStream_t st, double z0dz, double zd0, double dvv, float cw,
+template <bool HEL = false, typename TO>
+int run_cell_tma(int eff, const Geom& g, const float* in, TO* out, int nbatch, int nview, char* ws,
+                 const Layout& l, const ViewTables& vt, cudaStream_t st, double z0dz, double zd0, double dvv, float cw,
                  const float* zwt = nullptr) {
-    // FP32 images (also widened half-precision ones) go to any output type
-    if (!std::is_same<TI, float>::value && !std::is_same<TO, TI>::value && !std::is_same<TO, float>::value)
-        return -1;
+    using TI = float;  // half-precision images are widened first
     if (reinterpret_cast<uintptr_t>(in) % 16 != 0) return -1;
-    const CellPlan p = HEL ? plan_cell_helical(g) : plan_cell(g);
-    if (!p.ok || !encode_fn()) return -1;
+    const CellPlans plans = HEL ? plan_cell_helical(g) : plan_cell_shapes(g, 1 << 30);
+    if (!plans.base.ok || !encode_fn()) return -1;
+    const CellPlan& p = plans.launch;
     const size_t es = sizeof(TI);
     const int Hp = round_up(g.H, 8);
     TI* cols = reinterpret_cast<TI*>(ws + l.volT);
@@ -721,17 +773,18 @@ int run_cell_tma(int eff, const Geom& g, const TI* in, TO* out, int nbatch, int 
         rows = vr;
     }
     CUtensorMap mr, mc;
-    if (!encode_line_map(&mr, dtype_code<TI>(), rows, g.W, g.H, g.D, nbatch, Wp, p.BP, p.BZ) ||
-        !encode_line_map(&mc, dtype_code<TI>(), cols, g.H, g.W, g.D, nbatch, Hp, p.BP, p.BZ))
+    if (!encode_line_map(&mr, DT_F32, rows, g.W, g.H, g.D, nbatch, Wp, p.BP, p.BZ) ||
+        !encode_line_map(&mc, DT_F32, cols, g.H, g.W, g.D, nbatch, Hp, p.BP, p.BZ))
         return -1;
-    if (p.R == 16) {
-        if (eff == OP_A) return launch_cell_tma_mode<TI, TO, 16, OP_A, HEL>(g, p, mr, mc, rows, cols, Wp, Hp, out, nbatch, nview, vt, st, z0dz, zd0, dvv, cw, zwt);
-        if (eff == OP_BT) return launch_cell_tma_mode<TI, TO, 16, OP_BT, HEL>(g, p, mr, mc, rows, cols, Wp, Hp, out, nbatch, nview, vt, st, z0dz, zd0, dvv, cw, zwt);
-        return launch_cell_tma_mode<TI, TO, 16, OP_BWT, HEL>(g, p, mr, mc, rows, cols, Wp, Hp, out, nbatch, nview, vt, st, z0dz, zd0, dvv, cw, zwt);
-    }
-    if (eff == OP_A) return launch_cell_tma_mode<TI, TO, 8, OP_A, HEL>(g, p, mr, mc, rows, cols, Wp, Hp, out, nbatch, nview, vt, st, z0dz, zd0, dvv, cw, zwt);
-    if (eff == OP_BT) return launch_cell_tma_mode<TI, TO, 8, OP_BT, HEL>(g, p, mr, mc, rows, cols, Wp, Hp, out, nbatch, nview, vt, st, z0dz, zd0, dvv, cw, zwt);
-    return launch_cell_tma_mode<TI, TO, 8, OP_BWT, HEL>(g, p, mr, mc, rows, cols, Wp, Hp, out, nbatch, nview, vt, st, z0dz, zd0, dvv, cw, zwt);
+    auto launch = [&](auto r) -> int {
+        constexpr int R = decltype(r)::value;
+        if (eff == OP_A) return launch_cell_tma_mode<TO, R, OP_A, HEL>(g, p, mr, mc, rows, cols, Wp, Hp, out, nbatch, nview, vt, st, z0dz, zd0, dvv, cw, zwt);
+        if (eff == OP_BT) return launch_cell_tma_mode<TO, R, OP_BT, HEL>(g, p, mr, mc, rows, cols, Wp, Hp, out, nbatch, nview, vt, st, z0dz, zd0, dvv, cw, zwt);
+        return launch_cell_tma_mode<TO, R, OP_BWT, HEL>(g, p, mr, mc, rows, cols, Wp, Hp, out, nbatch, nview, vt, st, z0dz, zd0, dvv, cw, zwt);
+    };
+    if (p.R == 32) return launch(std::integral_constant<int, 32>{});
+    if (p.R == 16) return launch(std::integral_constant<int, 16>{});
+    return launch(std::integral_constant<int, 8>{});
 }
 
 template <typename TI, typename TO>
@@ -773,7 +826,7 @@ int run3d(int op, const Geom& g, const TI* in, TO* out, const float* ang, int nb
                 const size_t nt = vec ? (n + 7) / 8 : n;
                 widen_kernel<TI><<<(unsigned)((nt + 255) / 256), 256, 0, st>>>(in, vf, n, vec);
                 if (int e = check_cuda("widen")) return e;
-                rc = run_cell_tma<float, TO>(eff, g, vf, out, nbatch, nview, ws, l, vt, st, z0dz, zd0, dvv, cw);
+                rc = run_cell_tma(eff, g, vf, out, nbatch, nview, ws, l, vt, st, z0dz, zd0, dvv, cw);
             } else {
                 rc = run_cell_tma(eff, g, in, out, nbatch, nview, ws, l, vt, st, z0dz, zd0, dvv, cw);
             }
@@ -1125,7 +1178,7 @@ int helical(int op, const Geom& g, const HelOpts& o, const float* in, float* out
     const GeomF gf = make_geomf(g, 1);
     if (op == OP_A || op == OP_BT) {
         if (!g_force_plain) {
-            const int rc = run_cell_tma<float, float, true>(op, g, in, out, nbatch, nview, ws, hl.l, vt, st, z0dz,
+            const int rc = run_cell_tma<true>(op, g, in, out, nbatch, nview, ws, hl.l, vt, st, z0dz,
                                                               zd0, dvv, 0.0f);
             if (rc >= 0) return rc;
         }
@@ -1178,7 +1231,7 @@ int helical(int op, const Geom& g, const HelOpts& o, const float* in, float* out
         // per-voxel gather.  Without a TMA plan the per-voxel gather does all.
         int rc_tma = -1;
         if (!g_force_plain) {
-            rc_tma = run_cell_tma<float, float, true>(OP_BWT, g, imgs, out, nbatch, nview, ws, hl.l, vt, st, z0dz,
+            rc_tma = run_cell_tma<true>(OP_BWT, g, imgs, out, nbatch, nview, ws, hl.l, vt, st, z0dz,
                                                       zd0, dvv, (float)g.sod * (float)g.du, wtab_pad);
             if (rc_tma > 0) return rc_tma;
         }

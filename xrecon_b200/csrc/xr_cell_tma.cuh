@@ -88,26 +88,63 @@ __host__ __device__ inline CellWindow cell_window(const CellCtaGeo& c, const Vie
     return w;
 }
 
-// Stages of the line ring; the block barrier that frees a stage comes after
-// every XR_CELL_STAGES / 2 lines.
-#ifndef XR_CELL_STAGES
-#define XR_CELL_STAGES 4
-#endif
-constexpr int CELL_NS = XR_CELL_STAGES;
-static_assert(CELL_NS == 2 || CELL_NS == 4, "two or four stages");
-#ifndef XR_CELL_BATCH
-#define XR_CELL_BATCH (XR_CELL_STAGES / 2)  // lines per block barrier
-#endif
-static_assert(XR_CELL_BATCH >= 1 && XR_CELL_BATCH < XR_CELL_STAGES, "a barrier frees at most all but one stage");
+// Stages of the line ring; the block barrier that frees stages comes after
+// every NS / 2 lines.
+// Two stages leave shared memory for 16 warps per SM (what 128 registers a
+// thread allow) at every launch shape.
+constexpr int CELL_NS = 2;
 
-// After a wait gave up: only the last CELL_NS lines issued, up to `last`,
+// Rows of the fine walk that may be in flight at once.  The rows are
+// independent up to their sums, and the compiler would start them all before
+// it finishes any: three registers a row, 472 bytes of spills with 32 rows.
+// Every WALK_CHUNK rows the run's start is re-read from shared memory behind a
+// warp barrier, so that at most two chunks are open (64 views of the
+// 512 x 512 x 256 / 1024 x 256 scan, 32 rows a thread: chunks of 2 5.85 ms, 3 and
+// 4 5.75, 8 6.09; 16 rows a thread without chunks 7.43).
+constexpr int WALK_CHUNK = 4;
+
+// After a wait gave up: only the last NS lines issued, up to `last`,
 // may still have copies in flight (each earlier line's copy was seen to land
 // by the issuing thread before it issued the next line into that stage).
 // The issuing thread lets them land, or gives up once more, before the CTA
 // exits, which keeps its shared memory allocated until then.
+template <int NS>
 __device__ __noinline__ void drain_stages(uint64_t* bar, int last) {
-    for (int Lp = max(last - (CELL_NS - 1), 0); Lp <= last; ++Lp)
-        mbar_wait_bounded(&bar[Lp % CELL_NS], (unsigned)((Lp / CELL_NS) & 1));
+    for (int Lp = max(last - (NS - 1), 0); Lp <= last; ++Lp)
+        mbar_wait_bounded(&bar[Lp % NS], (unsigned)((Lp / NS) & 1));
+}
+
+// Walk of one column's R rows over one line from global memory, with bounds
+// checks: adds the row sums to out.  Out of line and rolled, so that it costs
+// the staged walk no registers and no code; `wz` (null: 1) weighs slice j by
+// wz[(j + 1) * nview].
+template <typename TI, int NB>
+__device__ __noinline__ void cell_walk_global(const TI* __restrict__ base, size_t plane, int D, double t0, float bf,
+                                              const float (&w)[NB], int np, const float* wz, int nview, int R, float* out) {
+    const double jf = floor(t0);
+    int j = (int)jf;
+    float pos = (float)(t0 - jf), jn = 1.0f;
+    const float f = pos;
+    auto band = [&]() -> float {
+        if ((unsigned)j >= (unsigned)D) return 0.0f;
+        const float v = band_at<TI, NB>(base + (size_t)j * plane, w, np);
+        return wz ? v * __ldg(wz + (size_t)(j + 1) * nview) : v;
+    };
+    float vj = band();
+#pragma unroll 1
+    for (int i = 0; i < R; ++i) {
+        const float top = fmaf(bf, (float)(i + 1), f);
+        float a = 0.0f;
+        while (jn < top) {
+            a = fmaf(jn - pos, vj, a);
+            pos = jn;
+            ++j;
+            jn += 1.0f;
+            vj = band();
+        }
+        if (top > pos) { a = fmaf(top - pos, vj, a); pos = top; }
+        out[i] += a;
+    }
 }
 
 // FINE: the geometry's detector rows are (nearly) all shorter than a voxel,
@@ -135,15 +172,16 @@ cell_tma3d_kernel(const Geom g, const ViewTables vt, const __grid_constant__ CUt
                   const double zd0_p, const double dvv, const float cw_p, const int BP, const int BZ,
                   const float* __restrict__ zwt) {
     constexpr bool ZW = HEL && MODE == OP_BWT;
+    constexpr int NS = CELL_NS, BATCH = NS / 2;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     // each stage starts on a 128-byte boundary (TMA destination alignment) and
     // holds BZ + 1 rows: the spare row absorbs the look-ahead read of the
     // branch-free walk (never used in a result)
     const int stage_elems = cell_stage_elems<TI>(BP, BZ);
     TI* stage = reinterpret_cast<TI*>(smem_raw);
-    uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw + (size_t)CELL_NS * stage_elems * sizeof(TI));
+    uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw + (size_t)NS * stage_elems * sizeof(TI));
     // window of every line of this CTA (computed once, below)
-    int4* wins = reinterpret_cast<int4*>(bar + CELL_NS);
+    int4* wins = reinterpret_cast<int4*>(bar + NS);
 
     const int lane = threadIdx.x, tid = threadIdx.y * 32 + threadIdx.x;
     const int Nu = g.Nu;
@@ -225,7 +263,7 @@ cell_tma3d_kernel(const Geom g, const ViewTables vt, const __grid_constant__ CUt
     __shared__ int s_abort;
     volatile int* abort = &s_abort;
     if (tid == 0) {
-        for (int i = 0; i < CELL_NS; ++i) mbar_init(&bar[i], 1);
+        for (int i = 0; i < NS; ++i) mbar_init(&bar[i], 1);
         fence_barrier_init();
         s_abort = 0;
     }
@@ -236,13 +274,18 @@ cell_tma3d_kernel(const Geom g, const ViewTables vt, const __grid_constant__ CUt
     }
     // The spare row BZ of each stage is never written by TMA; the look-ahead
     // read multiplies it by zero, so it must hold finite values (zeros).
-    for (int i = tid; i < CELL_NS * BP; i += blockDim.x * blockDim.y)
+    for (int i = tid; i < NS * BP; i += blockDim.x * blockDim.y)
         stage[(size_t)(i / BP) * stage_elems + (size_t)BZ * BP + (i % BP)] = TI(0.0f);
     __syncthreads();
     int last = -1;  // last line issued (issuing thread)
     if (tid == 0)
-        for (int L = 0; L < min(CELL_NS, nlines); ++L) issue(L, L), last = L;
+        for (int L = 0; L < min(NS, nlines); ++L) issue(L, L), last = L;
 
+    float cold[FINE ? R : 1];  // sums of cell_walk_global, in local memory
+#pragma unroll
+    for (int i = 0; i < (FINE ? R : 1); ++i) cold[i] = 0.0f;
+    __shared__ float s_fu[256];  // per thread, see WALK_CHUNK
+    const unsigned pitch_b = (unsigned)BP * (unsigned)sizeof(TI);
     float acc[R];
 #pragma unroll
     for (int i = 0; i < R; ++i) acc[i] = 0.0f;
@@ -293,8 +336,8 @@ cell_tma3d_kernel(const Geom g, const ViewTables vt, const __grid_constant__ CUt
     // read stays inside the staged windows, whatever they hold) so that all
     // threads meet every barrier; the results are dropped at the end.
     for (int L = 0; L < nlines; ++L) {
-        const int s = L % CELL_NS;
-        const unsigned parity = (unsigned)((L / CELL_NS) & 1);
+        const int s = L % NS;
+        const unsigned parity = (unsigned)((L / NS) & 1);
         mbar_wait_bounded(&bar[s], parity, abort);
         CellWindow win;
         {
@@ -302,25 +345,24 @@ cell_tma3d_kernel(const Geom g, const ViewTables vt, const __grid_constant__ CUt
             win.p0 = wi.x; win.z0 = wi.y; win.zlast = wi.z; win.empty = wi.w & 1; win.ok = wi.w >> 1;
         }
         if (active) {
-            const double pk = fma(bB0, (double)L, bA0);
-            const double pk1 = fma(bB1, (double)L, bA1);
+            const double dL = (double)L;
+            const double pk = fma(bB0, dL, bA0);
+            const double pk1 = fma(bB1, dL, bA1);
             const int pa = max((int)floor(pk), 0);
             const int pb = min((int)ceil(pk1) - 1, npix - 1);
+            const float u0 = (float)(pk - (double)pa), u1 = (float)(pk1 - (double)pa);
             const float Lf = (float)L;
-            const double t0 = fma(t0l, (double)L, t0c);
+            const double t0 = fma(t0l, dL, t0c);
+            const float t0f = (float)t0;
             const float bf = fmaf(btl, Lf, btc);
-            const bool live = !win.empty && (pa <= pb) && (bf > 1.0e-4f && bf < 1.0e4f) &&
-                              !(t0 + R * (double)bf <= 0.0 || t0 >= (double)g.D);
-            if (live) {
-                const double jf = floor(t0);
-                const int j0 = (int)jf;
-                const float f = (float)(t0 - jf);
+            const bool lit = !win.empty && (pa <= pb) && (bf > 1.0e-4f && bf < 1.0e4f) &&
+                              !(fmaf((float)R, bf, t0f) <= 0.0f || t0f >= (float)g.D);
+            if (lit) {
                 float lf = cw;
                 if (MODE == OP_A) {
                     const float qf = fmaf(ql, Lf, qc);
-                    lf = __fdividef(dpdz, qf * qf);
+                    lf = dpdz * rcp_fast(qf * qf);
                 }
-                const float u0 = (float)(pk - (double)pa), u1 = (float)(pk1 - (double)pa);
                 for (int pc = pa; pc <= pb; pc += NB) {
                     const int np = min(NB, pb - pc + 1);
                     const float off = (float)(pc - pa);
@@ -334,7 +376,6 @@ cell_tma3d_kernel(const Geom g, const ViewTables vt, const __grid_constant__ CUt
                         }
                         w[i] = wi;
                     }
-                    float pos = f, jn = 1.0f, vj;
                     if (win.ok && bf < 0.999f) {
                         // Rows shorter than a voxel: each row crosses at most
                         // one voxel boundary.  In window slice coordinates
@@ -346,26 +387,45 @@ cell_tma3d_kernel(const Geom g, const ViewTables vt, const __grid_constant__ CUt
                         //         + band(n) (u_{i+1} - max(n, u_i)).
                         // When the row does not cross, the first term is zero
                         // whatever band(n - 1) is, so each row forms one band
-                        // and keeps it for the next; floor is a conversion
-                        // to int and back (two issue slots; the rounding by
-                        // an FP32 add of 1.5 * 2^23 took four and made the
-                        // walk 5 % slower).  u is clamped to the staged
-                        // slices 0 .. win.zlast - win.z0 (slices -1 and D of
-                        // the volume arrive as zeros, and the window covers
-                        // every t of the CTA otherwise).
-                        const float fu = f + (float)(j0 - win.z0);
+                        // and keeps it for the next.  floor is an add of 1.5 *
+                        // 2^23 rounded down, whose bits times the stage's row
+                        // pitch, in modular arithmetic, are the slice's
+                        // offset: two FMA-pipe slots, where a conversion to
+                        // int and back took two on the quarter-rate
+                        // conversion pipe (44 % busy).  u is clamped to the
+                        // staged slices 0 .. win.zlast - win.z0 (slices -1
+                        // and D of the volume arrive as zeros, and the
+                        // window covers every t of the CTA otherwise).
+                        const unsigned live = __activemask();
+                        float fu = (float)(t0 - (double)win.z0), fu_next = fu;
+                        *(volatile float*)&s_fu[tid] = fu;
                         const float uhi = (float)(win.zlast - win.z0) + 0.999f;
-                        const TI* sb = stage + (size_t)s * stage_elems + XR_BOUND(pc - win.p0, 0, BP - np);
+                        const unsigned sb = (unsigned)(((size_t)s * stage_elems + XR_BOUND(pc - win.p0, 0, BP - np)) * sizeof(TI)) -
+                                            0x4B400000u * pitch_b;
                         auto slice_at = [&](float u, float& n) -> float {
-                            const int ri = __float2int_rd(u);
-                            n = (float)ri;
-                            return band_smem<TI, NB>(sb + XR_BOUND(ri, 0, BZ) * BP, w, np) * slice_w(win.z0 + ri);
+                            const float tr = __fadd_rd(u, 12582912.0f);
+                            n = tr - 12582912.0f;
+                            const unsigned off = (unsigned)__float_as_int(tr) * pitch_b + sb;
+#ifdef XR_DEBUG_BOUNDS
+                            const TI* q = reinterpret_cast<const TI*>(smem_raw + XR_BOUND((long long)off, 0, (long long)NS * stage_elems * (long long)sizeof(TI) - 4));
+#else
+                            const TI* q = reinterpret_cast<const TI*>(smem_raw + off);
+#endif
+                            return band_smem<TI, NB>(q, w, np) * slice_w(win.z0 + (__float_as_int(tr) - 0x4B400000));
                         };
                         float up = fminf(fmaxf(fu, 0.0f), uhi);
                         float np0;
                         float bp = slice_at(up, np0);
 #pragma unroll
                         for (int i = 0; i < R; ++i) {
+                            // a new chunk: fu comes back through memory, one
+                            // chunk ahead, which keeps the compiler from
+                            // starting the later rows now (see WALK_CHUNK)
+                            if (i % WALK_CHUNK == 0) {
+                                if (i) __syncwarp(live);
+                                fu = fu_next;
+                                fu_next = *(volatile float*)&s_fu[tid];
+                            }
                             const float u1 = fminf(fmaxf(fmaf(bf, (float)(i + 1), fu), 0.0f), uhi);
                             float n;
                             const float bn = slice_at(u1, n);
@@ -377,6 +437,10 @@ cell_tma3d_kernel(const Geom g, const ViewTables vt, const __grid_constant__ CUt
                             up = u1;
                         }
                     } else if (!FINE && win.ok) {
+                        const double jf = floor(t0);
+                        const int j0 = (int)jf;
+                        const float f = (float)(t0 - jf);
+                        float pos = f, jn = 1.0f, vj;
                         // Staged voxels win.z0 .. win.zlast; below the window a
                         // single virtual zero voxel ends at win.z0, past
                         // win.zlast the value is zero and the next boundary
@@ -413,44 +477,35 @@ cell_tma3d_kernel(const Geom g, const ViewTables vt, const __grid_constant__ CUt
                             acc[i] += a;
                         }
                     } else {
-                        // global fallback with bounds checks
+                        // rows of a voxel or more, or a window outside its box
                         const TI* base = fbb + (size_t)L * pitch + pc;
-                        int j = j0;
-                        vj = ((unsigned)j < (unsigned)g.D) ? band_at(base + (size_t)j * fb_plane, w, np) * slice_w(j) : 0.0f;
+                        if constexpr (FINE) {
+                            cell_walk_global<TI, NB>(base, fb_plane, g.D, t0, bf, w, np, ZW ? wz : nullptr, nview, R, cold);
+                        } else {
+                            float rows[R] = {};
+                            cell_walk_global<TI, NB>(base, fb_plane, g.D, t0, bf, w, np, ZW ? wz : nullptr, nview, R, rows);
 #pragma unroll
-                        for (int i = 0; i < R; ++i) {
-                            const float top = fmaf(bf, (float)(i + 1), f);
-                            float a = 0.0f;
-                            while (jn < top) {
-                                a = fmaf(jn - pos, vj, a);
-                                pos = jn;
-                                ++j;
-                                jn += 1.0f;
-                                vj = ((unsigned)j < (unsigned)g.D) ? band_at(base + (size_t)j * fb_plane, w, np) * slice_w(j) : 0.0f;
-                            }
-                            if (top > pos) { a = fmaf(top - pos, vj, a); pos = top; }
-                            acc[i] += a;
+                            for (int i = 0; i < R; ++i) acc[i] += rows[i];
                         }
                     }
                 }
             }
         }
         // every BATCH lines: all warps are done with those lines' stages,
-        // which take the lines CELL_NS further on
-        constexpr int BATCH = XR_CELL_BATCH;
+        // which take the lines NS further on
         if ((L + 1) % BATCH == 0) {
             __syncthreads();
             if (tid == 0 && !*abort) {
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 for (int j = L + 1 - BATCH; j <= L; ++j)
-                    if (j + CELL_NS < nlines) issue(j + CELL_NS, j % CELL_NS), last = j + CELL_NS;
+                    if (j + NS < nlines) issue(j + NS, j % NS), last = j + NS;
             }
         }
     }
     __syncthreads();
     // every wait ended before this barrier, so all threads read the same
     if (*abort) {
-        if (tid == 0) drain_stages(bar, last);
+        if (tid == 0) drain_stages<NS>(bar, last);
         return;
     }
 
@@ -466,7 +521,7 @@ cell_tma3d_kernel(const Geom g, const ViewTables vt, const __grid_constant__ CUt
     for (int i = 0; i < R; ++i) {
         const int r = r0 + i;
         if (r < g.Nv) {
-            float sv = acc[i];
+            float sv = FINE ? acc[i] + cold[i] : acc[i];
             if (MODE == OP_A) {
                 float zc = (float)(zd0 + (r + 0.5) * dvv) * M;
                 if (HEL) zc += vt.hel[v].zsrc;  // helical: the row's absolute z

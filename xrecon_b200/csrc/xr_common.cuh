@@ -153,6 +153,13 @@ template <> __device__ __forceinline__ void st<float>(float* p, float v) { *p = 
 template <> __device__ __forceinline__ void st<__nv_bfloat16>(__nv_bfloat16* p, float v) { *p = __float2bfloat16_rn(v); }
 template <> __device__ __forceinline__ void st<__half>(__half* p, float v) { *p = __float2half_rn(v); }
 
+// Store into an output of run-time type.
+__device__ __forceinline__ void st_dt(void* out, int dt, size_t i, float v) {
+    if (dt == DT_F32) st(static_cast<float*>(out) + i, v);
+    else if (dt == DT_BF16) st(static_cast<__nv_bfloat16*>(out) + i, v);
+    else st(static_cast<__half*>(out) + i, v);
+}
+
 // Hardware reciprocal (relative error 2^-23), one instruction: without the
 // denormal handling of __fdividef, whose operands here are lengths.
 __device__ __forceinline__ float rcp_fast(float x) {

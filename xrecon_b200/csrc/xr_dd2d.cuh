@@ -89,13 +89,6 @@ __device__ __forceinline__ Lanes<NB> ld_lanes(const float* p, size_t n, size_t i
     return r;
 }
 
-// Store into an output of run-time type.
-__device__ __forceinline__ void st_dt(void* out, int dt, size_t i, float v) {
-    if (dt == DT_F32) st(static_cast<float*>(out) + i, v);
-    else if (dt == DT_BF16) st(static_cast<__nv_bfloat16*>(out) + i, v);
-    else st(static_cast<__half*>(out) + i, v);
-}
-
 // ------------------------------------------------------------ preparation
 
 // Per-view tables and the input's second form in one launch (both small):
