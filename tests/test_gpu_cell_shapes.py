@@ -1,0 +1,33 @@
+"""The staged projection's launch shapes (rows per thread, warps per CTA, pixels
+per pass) against the FP64 oracle: detector heights on both sides of every
+shape, columns of under one and over two pixels, and a few lines with rows of
+more than a voxel, which leave the fine walk.
+
+Tolerance: 1e-5 relative L2, the bound of every operator against the oracle."""
+import numpy as np
+import pytest
+import torch
+
+from conftest import rel_l2
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("Nv", [1, 8, 9, 16, 17, 32, 33, 64, 65, 128, 129, 160])
+@pytest.mark.parametrize("du,dv", [(1.3, 1.0), (4.4, 1.0), (1.3, 1.52)])
+def test_projection_launch_shapes_match_the_oracle(cuda, Nv, du, dv):
+    from xrecon_b200 import _native
+    from xrecon_b200 import geometry as G
+    from xrecon_b200.backend import HostGeometry
+    D = max(4, int(Nv * 0.45))
+    geo = G.ConeBeam3d(G.Detector3d((45, Nv), (du, dv), (0.3, 0.2)), 200.0, 400.0, "flat")
+    opts = np.array(G.pack_options3d(G.Volume3d((26, 23, D), 1.0, (0.4, -0.2, 0.3)), geo), np.float32)
+    geom = HostGeometry(3, opts.tolist()).struct
+    plan = _native.cell_plan(geom)
+    assert plan["ok"] and plan["fine"]
+    ang = np.array([0.03, 0.7, np.pi / 4, 2.2, 3.9, 5.6], np.float32)
+    img = np.random.default_rng(Nv).random((1, 2, D, 23, 26)).astype(np.float32)
+    for op in ("A", "BT", "BWT"):
+        got = _native.apply(3, op, torch.from_numpy(img).to(cuda), geom, torch.from_numpy(ang).to(cuda))
+        assert rel_l2(got.cpu().numpy(), O.dd3d(op, img, opts, ang)) < 1e-5, op
