@@ -402,7 +402,7 @@ Layout layout(int dim3d, int op, const Geom& g, int nbatch, int nview, int dtype
     // the plain kernels' pre-scaled cone A^T sinogram reuses the region
     l.sinoS = o;
     if (dim3d && (eff == OP_AT || eff == OP_B || eff == OP_BW))
-        o = align256(o + (size_t)nbatch * V * (g.Nv + 2) * g.Nu * sizeof(float2));
+        o = align256(o + (size_t)nbatch * V * (g.Nv + 2) * tab_pitch(g.Nu) * sizeof(float2));
     // the staged prefix gather's per-CTA flags (views left to its fallback)
     l.pfxF = o;
     if (l.has_pfx)
@@ -512,7 +512,7 @@ PfxStagePlan plan_pfx_stage(const Geom& g) {
         if (it != cache.end()) return it->second;
     }
     PfxStagePlan p{false, 0, 0};
-    if ((g.type == GEO_FLAT || g.type == GEO_PARALLEL || g.type == GEO_ARC) && g.Nu % 2 == 0 &&
+    if ((g.type == GEO_FLAT || g.type == GEO_PARALLEL || g.type == GEO_ARC) &&
         (g.type != GEO_ARC || XR_GUESS_ATAN_ERR / g.du < 0.25)) {
         const GeomF gf = make_geomf(g, 1);
         double zd0, dvv, z0dz;
@@ -649,7 +649,8 @@ bool encode_table_map(CUtensorMap* m, const float2* tab, const Geom& g, int nbv,
     EncodeTiledFn fn = encode_fn();
     if (!fn) return false;
     cuuint64_t dims[3] = {(cuuint64_t)g.Nu, (cuuint64_t)(g.Nv + 2), (cuuint64_t)nbv};
-    cuuint64_t strides[2] = {(cuuint64_t)g.Nu * 8, (cuuint64_t)g.Nu * 8 * (g.Nv + 2)};
+    const cuuint64_t pitch = (cuuint64_t)tab_pitch(g.Nu) * 8;
+    cuuint64_t strides[2] = {pitch, pitch * (g.Nv + 2)};
     cuuint32_t box[3] = {(cuuint32_t)BC, (cuuint32_t)BR, 1u};
     cuuint32_t estr[3] = {1u, 1u, 1u};
     const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, const_cast<float2*>(tab), dims, strides, box, estr,
@@ -862,7 +863,7 @@ int run3d(int op, const Geom& g, const TI* in, TO* out, const float* ang, int nb
     const GeomF gf = make_geomf(g, 1);
     const float atconst = (float)(g.dx * g.dy * g.dz / (g.du * g.dv));
     // the prefix kernel addresses one view's table with 32-bit byte offsets
-    const bool prefix_ok = (double)(g.Nv + 2) * g.Nu * sizeof(float2) < 2147483648.0;
+    const bool prefix_ok = (double)(g.Nv + 2) * tab_pitch(g.Nu) * sizeof(float2) < 2147483648.0;
     if (!g_force_plain && prefix_ok) {
         float2* tab = reinterpret_cast<float2*>(ws + l.sinoS);
         const int nbv = nbatch * nview;
@@ -1202,7 +1203,7 @@ int helical(int op, const Geom& g, const HelOpts& o, const float* in, float* out
         }
         return XR_OK;
     }
-    if ((double)(g.Nv + 2) * g.Nu * sizeof(float2) >= 2147483648.0)
+    if ((double)(g.Nv + 2) * tab_pitch(g.Nu) * sizeof(float2) >= 2147483648.0)
         return fail(XR_ERR_UNSUPPORTED, "detector of %d x %d cells too large for one view's row table", g.Nu, g.Nv);
     HelZ* zw = reinterpret_cast<HelZ*>(ws + hl.zw);
     HelScanF* scan = reinterpret_cast<HelScanF*>(ws + hl.scan);
@@ -1538,7 +1539,7 @@ int xr_pfx_stage_plan(const xr_geom3d* geom, int* ok, int* box_cols, int* box_ro
     const xr::Geom g = xr::geom_from(geom);
     if (int rc = xr::validate(g, 1, 0, 1, 1)) return rc;
     const xr::PfxStagePlan p = xr::plan_pfx_stage(g);
-    *ok = p.ok;
+    *ok = p.ok && g.Nu % 2 == 0;  // the box of an odd count is that of its padded tables
     *box_cols = p.BC;
     *box_rows = p.BR;
     return XR_OK;

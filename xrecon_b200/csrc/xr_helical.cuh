@@ -495,7 +495,7 @@ hel_wbp_kernel(const Geom g, const GeomF gf, const ViewTables vt, const HelOpts 
     const float row_off = 0.5f * (float)g.Nv - 0.5f;
     if (ix >= g.W || iy >= g.H || j0 >= g.D) return;
     const int Nu = g.Nu, Nv = g.Nv;
-    const size_t vstride = (size_t)(Nv + 2) * Nu;
+    const size_t vstride = (size_t)(Nv + 2) * tab_pitch(Nu);
     const float px = hw_px(g, ix), py = hw_py(g, iy);
     const HelScanF s = *scan;
     float acc[R], valid[R];
@@ -601,7 +601,7 @@ hel_wbp_kernel(const Geom g, const GeomF gf, const ViewTables vt, const HelOpts 
         const int kb = min(Nu - 1, (int)floorf(hi + margin));
         if (ka > kb) continue;
         const char* __restrict__ tvb = reinterpret_cast<const char*>(tab + ((size_t)b * nview + v) * vstride);
-        const unsigned Nu8 = (unsigned)Nu * 8u;
+        const unsigned Nu8 = (unsigned)tab_pitch(Nu) * 8u;
         // Boundaries relative to the pixel: boundary ka in FP64, the next ones
         // by the columns' widths on this line in FP32; the run's row offset
         // and rows per voxel in FP64 at the first column, at the next ones

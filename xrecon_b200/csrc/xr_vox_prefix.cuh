@@ -29,6 +29,10 @@
 
 namespace xr {
 
+// Columns of a table row in memory: even, so that every row starts on the 16
+// bytes a TMA copy needs.
+__host__ __device__ inline int tab_pitch(int Nu) { return (Nu + 1) & ~1; }
+
 // One thread per (batch element x view, physical column).  MODE OP_AT with a
 // cone geometry folds the projection's cell scale s_A(k, r) into y, as
 // prescale_at3d_kernel does.
@@ -42,7 +46,8 @@ row_prefix3d_kernel(const Geom g, const ViewTables vt, const TI* __restrict__ in
     for (int bv = blockIdx.y; bv < nbv; bv += gridDim.y) {
         const int v = bv % nview;
         const TI* __restrict__ src = in + (size_t)bv * Nv * Nu + c;
-        float2* __restrict__ dst = tab + (size_t)bv * (Nv + 2) * Nu + c;
+        const int pitch = tab_pitch(Nu);
+        float2* __restrict__ dst = tab + (size_t)bv * (Nv + 2) * pitch + c;
         float E = 1.0f, F = 0.0f, M = 0.0f;
         double zd0 = zd0_p;
         float zsrc = 0.0f;
@@ -65,10 +70,10 @@ row_prefix3d_kernel(const Geom g, const ViewTables vt, const TI* __restrict__ in
         dst[0] = make_float2((float)run, 0.0f);
         for (int r = 0; r < Nv; ++r) {
             const float y = value(r);
-            dst[(size_t)(r + 1) * Nu] = make_float2((float)(run + 0.5 * (double)y), y);
+            dst[(size_t)(r + 1) * pitch] = make_float2((float)(run + 0.5 * (double)y), y);
             run += (double)y;
         }
-        dst[(size_t)(Nv + 1) * Nu] = make_float2((float)run, 0.0f);
+        dst[(size_t)(Nv + 1) * pitch] = make_float2((float)run, 0.0f);
     }
 }
 
@@ -120,8 +125,8 @@ vox_prefix3d_kernel(const Geom g, const GeomF gf, const ViewTables vt, const flo
     const int j0 = zg * R;
     if (ix >= g.W || iy >= g.H || j0 >= g.D) return;
     const int Nu = g.Nu, Nv = g.Nv;
-    const unsigned Nu8 = (unsigned)Nu * 8u;
-    const size_t vstride = (size_t)(Nv + 2) * Nu;
+    const unsigned Nu8 = (unsigned)tab_pitch(Nu) * 8u;
+    const size_t vstride = (size_t)(Nv + 2) * tab_pitch(Nu);
     const float2* __restrict__ tb = tab + (size_t)b * nview * vstride;
     double zs = (double)j0 + z0dz;  // run bottom, in voxel units from z = 0
     double zoffh = -zd0 / dvv - 0.5;  // u0 = zs * (rows per voxel) + zoffh

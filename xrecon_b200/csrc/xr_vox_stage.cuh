@@ -201,8 +201,8 @@ vox_stage3d_kernel(const Geom g, const GeomF gf, const ViewTables vt, const __gr
     if (FALLBACK && unfit[cta] == 0) return;  // CTA-uniform
 
     const int Nu = g.Nu, Nv = g.Nv;
-    const unsigned Nu8 = (unsigned)Nu * 8u;
-    const size_t vstride = (size_t)(Nv + 2) * Nu;
+    const unsigned Nu8 = (unsigned)tab_pitch(Nu) * 8u;
+    const size_t vstride = (size_t)(Nv + 2) * tab_pitch(Nu);
     const float2* __restrict__ tb = tab + (size_t)b * nview * vstride;
     const double zs0 = (double)j0 + z0dz;  // run bottom, in voxel units from z = 0
     const double zoffh0 = -zd0 / dvv - 0.5;  // u0 = zs * (rows per voxel) + zoffh
