@@ -168,6 +168,13 @@ __device__ __forceinline__ float rcp_fast(float x) {
     return r;
 }
 
+// 1 / x in FP64 to about 2^-46: the hardware reciprocal and one Newton step (the
+// correctly rounded one is a dozen instructions).
+__device__ __forceinline__ double drcp_fast(double x) {
+    const double r = (double)rcp_fast((float)x);
+    return fma(r, fma(-x, r, 1.0), r);
+}
+
 // ---------------------------------------------------------------- geometry
 
 // Axis decision and traversal order exactly as the reference CPU path takes
@@ -466,13 +473,13 @@ __device__ __forceinline__ void line_point(const Geom& g, const ViewHdr& h, int 
 __device__ __forceinline__ float fbp_weight(const Geom& g, const ViewHdr& h, float px, float py) {
     if (g.type == GEO_FLAT) {
         const float R = (float)g.sod;
-        const float d = __fdividef((float)h.sx * px + (float)h.sy * py, R);
-        const float den = R - d;
-        return __fdividef(R * R, den * den);
+        // (R / (R - (s . p) / R))^2 with s = R (-sin, cos)
+        const float m = R * rcp_fast(fmaf(px, h.sf, fmaf(-py, h.cf, R)));
+        return m * m;
     }
     if (g.type == GEO_ARC) {
-        const float ex = (float)h.sx - px, ey = (float)h.sy - py;
-        return __fdividef(1.0f, ex * ex + ey * ey);
+        const float ex = h.sxr - px, ey = h.syr - py;
+        return rcp_fast(ex * ex + ey * ey);
     }
     return 1.0f;
 }

@@ -583,17 +583,17 @@ hel_wbp_kernel(const Geom g, const GeomF gf, const ViewTables vt, const HelOpts 
         const double zs = (double)j0 + hv.z0dz;
         const double zoffh = hv.zoffh;
         const double q = fma(h.q1, (double)L, h.q0);
-        const double mvdv = __drcp_rn(q * dvv);
+        const double mvdv = drcp_fast(q * dvv);
         // column width SOD du over the squared source distance
         const float lf = __fdiv_rn(s.cwW, __fadd_rn(__fmul_rn(rx, rx), __fmul_rn(ry, ry)));
         const float margin = 0.5f + XR_GUESS_ATAN_ERR * hv.inv_du;
-        const float sf = (float)h.s, cf = (float)h.c;
+        const float sf = h.sf, cf = h.cf;
         // one guess at the pixel centre and a bound on the footprint's
         // half-width: the pixel's edge segment on this line (half-length a,
         // at rxy from the source) spans at most a / (rxy - a) rad each side
         const float kc = col_guess_fast(gf, h, sf, cf, h.dcx, h.dcy, px, py, hv.inv_du);
         const float ha = 0.5f * (h.use_x ? gf.dx : gf.dy);
-        const float hw = __fdividef(ha, fmaxf(rxy - ha, ha)) * hv.inv_du * 1.001f;
+        const float hw = ha * rcp_fast(fmaxf(rxy - ha, ha)) * hv.inv_du * 1.001f;
         const float kf0 = kc - hw, kf1 = kc + hw;
         const float lo = fmaxf(fminf(fminf(kf0, kf1), (float)Nu + 2.0f), -2.0f);
         const float hi = fmaxf(fminf(fmaxf(kf0, kf1), (float)Nu + 2.0f), -2.0f);
@@ -643,7 +643,7 @@ hel_wbp_kernel(const Geom g, const GeomF gf, const ViewTables vt, const HelOpts 
                 if (fib < 4096.0f && ub < (float)Nv - 0.5f && fmaf((float)R, fib, ub) > -0.5f) {
                     const int col = keep ? k : Nu - 1 - k;
                     const char* cb = reinterpret_cast<const char*>(rb + (uintptr_t)col * 8u);
-                    const float wk = __fdividef(wf * lf, fib);
+                    const float wk = wf * lf * rcp_fast(fib);
                     float gprev = 0.0f;
 #pragma unroll
                     for (int i = 0; i <= R; ++i) {

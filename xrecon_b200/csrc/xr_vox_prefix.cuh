@@ -86,10 +86,10 @@ __device__ __forceinline__ float col_guess_fast(const GeomF& gf, const ViewHdr& 
     float sg;
     if (gf.type == GEO_FLAT) {
         const float R = gf.sod;
-        const float u = __fdividef(R * (x * c + y * s), R + x * s - y * c);
+        const float u = R * (x * c + y * s) * rcp_fast(R + x * s - y * c);
         sg = (u * gf.inv_uscale - gf.shu) * inv_du;
     } else if (gf.type == GEO_ARC) {
-        const float ex = x - (float)h.sx, ey = y - (float)h.sy;
+        const float ex = x - h.sxr, ey = y - h.syr;
         sg = guess_atan2f(dcx * ey - dcy * ex, dcx * ex + dcy * ey) * inv_du;
     } else {
         sg = (x * c + y * s - gf.shu) * inv_du;
@@ -171,17 +171,17 @@ vox_prefix3d_kernel(const Geom g, const GeomF gf, const ViewTables vt, const flo
             py = ya + 0.5f * gf.dy;
         }
         const double q = fma(h.q1, (double)L, h.q0);
-        const double mvdv = __drcp_rn(q * dvv);  // rows per voxel = mvdv * colR[k]
+        const double mvdv = drcp_fast(q * dvv);  // rows per voxel = mvdv * colR[k]
         float lf;
         if (MODE == OP_AT) {
             if (g.type == GEO_PARALLEL) lf = atconst;
-            else { const float qf = (float)q; lf = (float)h.dpix * dpdz / (qf * qf); }
+            else { const float qf = (float)q; lf = (h.use_x ? gf.dx : gf.dy) * dpdz * rcp_fast(qf * qf); }
         } else {
             lf = cwv;
             if (MODE == OP_BW) lf *= fbp_weight(g, h, px, py);
         }
         lf *= oscale;
-        const float sf = (float)h.s, cf = (float)h.c;
+        const float sf = h.sf, cf = h.cf;
         const float dcx = h.dcx, dcy = h.dcy;
         float kf0, kf1;
         if (CHAIN) {  // arc detector (the other instantiations keep two guesses: fewer live registers)
@@ -190,10 +190,10 @@ vox_prefix3d_kernel(const Geom g, const GeomF gf, const ViewTables vt, const flo
             // a, distance r from the source) spans at most a / (r - a) rad
             // each side of the centre
             const float kc = col_guess_fast(gf, h, sf, cf, dcx, dcy, px, py, inv_du);
-            const float ex = px - (float)h.sx, ey = py - (float)h.sy;
+            const float ex = px - h.sxr, ey = py - h.syr;
             const float a = 0.5f * (h.use_x ? gf.dx : gf.dy);
             const float r2 = fmaf(ex, ex, ey * ey);
-            const float hw = __fdividef(a, fmaxf(r2 * rsqrtf(r2) - a, a)) * inv_du * 1.001f;
+            const float hw = a * rcp_fast(fmaxf(r2 * rsqrtf(r2) - a, a)) * inv_du * 1.001f;
             kf0 = kc - hw;
             kf1 = kc + hw;
         } else {
@@ -227,7 +227,7 @@ vox_prefix3d_kernel(const Geom g, const GeomF gf, const ViewTables vt, const flo
         const float4* __restrict__ ea = nullptr;
         if (CHAIN) {
             ea = vt.arc + 2 * (size_t)v * (Nu + 1);
-            qd = __fdividef((float)q, h.use_x ? gf.dx : gf.dy);  // pixels per axis unit on this line (scales the chain's small offsets)
+            qd = (float)q * rcp_fast(h.use_x ? gf.dx : gf.dy);  // pixels per axis unit on this line (scales the chain's small offsets)
             ch.start(ea, k, keep, gf.du);
             float d = ch.next_linear(ea, k + 1);
             if (k + 1 == Nu) d = fminf(d, 0.0f);  // the detector's end
@@ -282,7 +282,7 @@ vox_prefix3d_kernel(const Geom g, const GeomF gf, const ViewTables vt, const flo
                     return __ldg(reinterpret_cast<const float2*>(cb + (size_t)(unsigned)__float_as_int(tr) * Nu8));
                 };
 #endif
-                const float wk = __fdividef(wf * lf, fib);
+                const float wk = wf * lf * rcp_fast(fib);
                 // rows the run reaches, inside [0, Nv - 1] in every active lane?
                 const bool inside = (ub >= 0.0f) && (ut <= (float)(Nv - 1));
                 float gprev = 0.0f;

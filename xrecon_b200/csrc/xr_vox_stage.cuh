@@ -115,7 +115,7 @@ __device__ inline int4 pfx_window(const Geom& g, const GeomF& gf, const ViewTabl
         yl = gf.y0 + (float)(g.H - 1 - iye) * gf.dy;
         yh = gf.y0 + (float)(g.H - iy0) * gf.dy;
     }
-    const float sf = (float)h.s, cf = (float)h.c;
+    const float sf = h.sf, cf = h.cf;
     float gmin = 3.0e38f, gmax = -3.0e38f;
     auto corner = [&](float x, float y) {
         const float k = col_guess_fast(gf, h, sf, cf, h.dcx, h.dcy, x, y, inv_du);
@@ -292,25 +292,25 @@ vox_stage3d_kernel(const Geom g, const GeomF gf, const ViewTables vt, const __gr
                 py = ya + 0.5f * gf.dy;
             }
             const double q = fma(h.q1, (double)L, h.q0);
-            const double mvdv = __drcp_rn(q * dvv);  // rows per voxel = mvdv * colR[k]
+            const double mvdv = drcp_fast(q * dvv);  // rows per voxel = mvdv * colR[k]
             float lf;
             if (MODE == OP_AT) {
                 if (g.type == GEO_PARALLEL) lf = atconst;
-                else { const float qf = (float)q; lf = (float)h.dpix * dpdz / (qf * qf); }
+                else { const float qf = (float)q; lf = (h.use_x ? gf.dx : gf.dy) * dpdz * rcp_fast(qf * qf); }
             } else {
                 lf = cwv;
                 if (MODE == OP_BW) lf *= fbp_weight(g, h, px, py);
             }
             lf *= oscale;
-            const float sf = (float)h.s, cf = (float)h.c;
+            const float sf = h.sf, cf = h.cf;
             float kf0, kf1;
             if (CHAIN) {
                 // one guess at the pixel centre and the footprint's half-width bound
                 const float kc = col_guess_fast(gf, h, sf, cf, h.dcx, h.dcy, px, py, inv_du);
-                const float ex = px - (float)h.sx, ey = py - (float)h.sy;
+                const float ex = px - h.sxr, ey = py - h.syr;
                 const float a = 0.5f * (h.use_x ? gf.dx : gf.dy);
                 const float r2 = fmaf(ex, ex, ey * ey);
-                const float hw = __fdividef(a, fmaxf(r2 * rsqrtf(r2) - a, a)) * inv_du * 1.001f;
+                const float hw = a * rcp_fast(fmaxf(r2 * rsqrtf(r2) - a, a)) * inv_du * 1.001f;
                 kf0 = kc - hw;
                 kf1 = kc + hw;
             } else {
@@ -347,7 +347,7 @@ vox_stage3d_kernel(const Geom g, const GeomF gf, const ViewTables vt, const __gr
             const float4* __restrict__ ea = nullptr;
             if (CHAIN) {
                 ea = vt.arc + 2 * (size_t)v * (Nu + 1);
-                qd = __fdividef((float)q, h.use_x ? gf.dx : gf.dy);  // pixels per axis unit on this line
+                qd = (float)q * rcp_fast(h.use_x ? gf.dx : gf.dy);  // pixels per axis unit on this line
                 ch.start(ea, k, keep, gf.du);
                 float d = ch.next_linear(ea, k + 1);
                 if (k + 1 == Nu) d = fminf(d, 0.0f);  // the detector's end
@@ -392,7 +392,7 @@ vox_stage3d_kernel(const Geom g, const GeomF gf, const ViewTables vt, const __gr
                         return *reinterpret_cast<const float2*>(sbase + off);
 #endif
                     };
-                    const float wk = __fdividef(wf * lf, fib);
+                    const float wk = wf * lf * rcp_fast(fib);
                     const bool inside = (ub >= in_lo) && (ut <= in_hi);
                     float gprev = 0.0f;
                     if (__all_sync(__activemask(), inside)) {
