@@ -118,7 +118,7 @@ template <typename TO, int R, int NWY, int MODE, bool HEL = false, bool CHAIN = 
 __global__ void __launch_bounds__(32 * NWY, XR_PFX_MINB)
 vox_prefix3d_kernel(const Geom g, const GeomF gf, const ViewTables vt, const float2* __restrict__ tab,
                     TO* __restrict__ vol, const int nview, const int nzg, const double z0dz, const double zd0,
-                    const double dvv, const float cw, const float atconst, const float oscale) {
+                    const double dvv, const float cw, const float atconst, const float oscale, const int CS) {
     const int ix = blockIdx.x * 32 + threadIdx.x;
     const int iy = blockIdx.y * NWY + threadIdx.y;
     const int zg = blockIdx.z % nzg, b = blockIdx.z / nzg;
@@ -141,7 +141,12 @@ vox_prefix3d_kernel(const Geom g, const GeomF gf, const ViewTables vt, const flo
 #pragma unroll
     for (int i = 0; i < R; ++i) acc[i] = 0.0f;
 
-    for (int v = 0; v < nview; ++v) {
+    // CS > 1: the views' sums taken as the staged gather takes them when it
+    // splits them over CS CTAs (views r, r + CS, ... first, then over r)
+    float sums[R];
+#pragma unroll 1
+    for (int r = 0; r < CS; ++r) {
+    for (int v = r; v < nview; v += CS) {
         const ViewHdr& h = vt.hdr[v];
         const int keep = h.keep;
         float cwv = cw;
@@ -340,6 +345,13 @@ vox_prefix3d_kernel(const Geom g, const GeomF gf, const ViewTables vt, const flo
                 pk1 = fmaf(d, qd, pd);
             }
         }
+    }
+    if (CS == 1) break;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        sums[i] = r ? sums[i] + acc[i] : acc[i];
+        acc[i] = r + 1 < CS ? 0.0f : sums[i];
+    }
     }
 #pragma unroll
     for (int i = 0; i < R; ++i) {

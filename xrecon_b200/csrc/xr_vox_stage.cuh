@@ -39,6 +39,8 @@
 // double-buffered table in shared memory.
 #pragma once
 
+#include <cooperative_groups.h>
+
 #include "xr_vox_prefix.cuh"
 #include "xr_tma.cuh"
 
@@ -62,6 +64,12 @@ __host__ __device__ inline size_t pfx_stage_bytes(int BC, int BR) {
 // Dynamic shared memory of the staged kernel: window table, barriers, ring.
 __host__ __device__ inline size_t pfx_stage_smem(int BC, int BR) {
     return 2 * PS_WCH * sizeof(int4) + 128 + PS_NS * pfx_stage_bytes(BC, BR);
+}
+// The same when a cluster splits the views: the ring also holds the CTA's
+// sums, R floats per thread.
+__host__ __device__ inline size_t pfx_split_smem(int BC, int BR, int R) {
+    const size_t ring = PS_NS * pfx_stage_bytes(BC, BR), sums = (size_t)PS_T * PS_T * R * sizeof(float);
+    return 2 * PS_WCH * sizeof(int4) + 128 + (ring > sums ? ring : sums);
 }
 
 // Box of view v for the CTA at tile (ix0, iy0) and z-run bottom zs:
@@ -179,12 +187,16 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
 // elements, box {BC, BR, 1}.  unfit[cta]: set by the staged launch when it
 // skipped a view; the FALLBACK launch does only those CTAs' skipped views,
 // adding to what the staged launch stored.
+// CS > 1 (staged launch only): the CTAs of a cluster along z share a tile, the
+// CTA of rank r taking views r, r + CS, ..., and add their sums through
+// distributed shared memory in rank order: a grid of a few waves then ends
+// without a nearly empty one.
 template <typename TO, int R, int MODE, bool FALLBACK, bool HEL = false, bool CHAIN = false>
 __global__ void __launch_bounds__(PS_T * PS_T, XR_PFXS_MINB)
 vox_stage3d_kernel(const Geom g, const GeomF gf, const ViewTables vt, const __grid_constant__ CUtensorMap map,
                    const float2* __restrict__ tab, TO* __restrict__ vol, int* __restrict__ unfit, const int nview,
                    const int nzg, const double z0dz, const double zd0, const double dvv, const float cw,
-                   const float atconst, const float oscale, const int BC, const int BR) {
+                   const float atconst, const float oscale, const int BC, const int BR, const int CS) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     int4* wins = reinterpret_cast<int4*>(smem_raw);
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw + 2 * PS_WCH * sizeof(int4));
@@ -194,10 +206,12 @@ vox_stage3d_kernel(const Geom g, const GeomF gf, const ViewTables vt, const __gr
     const int tid = threadIdx.x;
     const int ix0 = blockIdx.x * PS_T, iy0 = blockIdx.y * PS_T;
     const int ix = ix0 + (tid % PS_T), iy = iy0 + (tid / PS_T);
-    const int zg = blockIdx.z % nzg, b = blockIdx.z / nzg;
+    const int zi = blockIdx.z / CS, rank = blockIdx.z % CS;
+    const int zg = zi % nzg, b = zi / nzg;
     const int j0 = zg * R;
     const bool active = ix < g.W && iy < g.H && j0 < g.D;
-    const unsigned cta = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
+    const unsigned cta = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * zi);
+    const int nloc = (nview - rank + CS - 1) / CS;  // this CTA's views: rank + CS i, i < nloc
     if (FALLBACK && unfit[cta] == 0) return;  // CTA-uniform
 
     const int Nu = g.Nu, Nv = g.Nv;
@@ -219,33 +233,34 @@ vox_stage3d_kernel(const Geom g, const GeomF gf, const ViewTables vt, const __gr
         s_abort = 0;
         s_unfit = 0;
     }
-    auto windows = [&](int vbase) {
-        if (tid < PS_WCH && vbase + tid < nview) {
-            const int4 w = pfx_window<HEL, CHAIN>(g, gf, vt, vbase + tid, ix0, iy0, j0, zs0, zoffh0, dvv, R, BC, BR);
-            wins[((vbase / PS_WCH) & 1) * PS_WCH + tid] = w;
+    // windows and stages go by the CTA's own view count i
+    auto windows = [&](int ibase) {
+        if (tid < PS_WCH && ibase + tid < nloc) {
+            const int4 w = pfx_window<HEL, CHAIN>(g, gf, vt, rank + (ibase + tid) * CS, ix0, iy0, j0, zs0, zoffh0, dvv, R, BC, BR);
+            wins[((ibase / PS_WCH) & 1) * PS_WCH + tid] = w;
             if (w.x < 0) s_unfit = 1;
         }
     };
-    auto window_of = [&](int v) { return wins[((v / PS_WCH) & 1) * PS_WCH + v % PS_WCH]; };
+    auto window_of = [&](int i) { return wins[((i / PS_WCH) & 1) * PS_WCH + i % PS_WCH]; };
     windows(0);
     __syncthreads();
 
     // test hook: arm the barrier for a box but issue no copy
     const bool stall = (*(volatile unsigned*)&g_test_hooks & XR_HOOK_TMA_STALL) != 0;
     const unsigned box_bytes = (unsigned)((size_t)BC * BR * sizeof(float2));
-    auto issue = [&](int v) {
-        const int4 w = window_of(v);
-        uint64_t* br = &bar[v % PS_NS];
+    auto issue = [&](int i) {
+        const int4 w = window_of(i);
+        uint64_t* br = &bar[i % PS_NS];
         if (w.x >= 0 && w.z <= w.w) {
             mbar_arrive_expect_tx(br, box_bytes);
-            if (!stall) tma_load_3d(stages + (size_t)(v % PS_NS) * stage_bytes, &map, w.x, w.y, b * nview + v, br);
+            if (!stall) tma_load_3d(stages + (size_t)(i % PS_NS) * stage_bytes, &map, w.x, w.y, b * nview + rank + i * CS, br);
         } else {
             asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(br)) : "memory");
         }
     };
     int last = -1;  // last view issued (issuing thread)
     if (!FALLBACK && tid == 0)
-        for (int v = 0; v < min(PS_NS, nview); ++v) issue(v), last = v;
+        for (int i = 0; i < min(PS_NS, nloc); ++i) issue(i), last = i;
 
     float acc[R];
 #pragma unroll
@@ -256,10 +271,11 @@ vox_stage3d_kernel(const Geom g, const GeomF gf, const ViewTables vt, const __gr
             if (j0 + i < g.D) acc[i] = ld(vol + (((size_t)b * g.D + j0 + i) * g.H + iy) * g.W + ix);
     }
 
-    for (int v = 0; v < nview; ++v) {
-        const int4 w = window_of(v);
+    for (int vi = 0; vi < nloc; ++vi) {
+        const int v = rank + vi * CS;
+        const int4 w = window_of(vi);
         const bool mine = FALLBACK ? (w.x < 0) : (w.x >= 0 && w.z <= w.w);
-        if (!FALLBACK && mine) mbar_wait_bounded(&bar[v % PS_NS], (unsigned)((v / PS_NS) & 1), abort);
+        if (!FALLBACK && mine) mbar_wait_bounded(&bar[vi % PS_NS], (unsigned)((vi / PS_NS) & 1), abort);
         if (mine && active && !(!FALLBACK && *abort)) do {
             const ViewHdr& h = vt.hdr[v];
             const int keep = h.keep;
@@ -367,7 +383,7 @@ vox_stage3d_kernel(const Geom g, const GeomF gf, const ViewTables vt, const __gr
             // the sum is the entry's offset); fallback, the global table.
             const unsigned P = FALLBACK ? Nu8 : (unsigned)BC * 8u;
             const unsigned rb32 = (unsigned)(r0 + 1 - (FALLBACK ? 0 : w.y)) * P - 0x4B400000u * P;
-            const unsigned char* sbase = stages + (size_t)(v % PS_NS) * stage_bytes;
+            const unsigned char* sbase = stages + (size_t)(vi % PS_NS) * stage_bytes;
             const char* __restrict__ tvb = reinterpret_cast<const char*>(tb + (size_t)v * vstride);
             for (;;) {
                 const float wf = fminf(1.0f, pk1) - fmaxf(0.0f, pkl);
@@ -450,37 +466,64 @@ vox_stage3d_kernel(const Geom g, const GeomF gf, const ViewTables vt, const __gr
             }
         } while (false);
         if (!FALLBACK) {
-            // all threads are done with stage v % PS_NS: it takes view v + PS_NS
+            // all threads are done with stage vi % PS_NS: it takes view vi + PS_NS
             __syncthreads();
-            const int vn = v + PS_NS;
-            if (vn < nview && vn % PS_WCH == 0) {
+            const int vn = vi + PS_NS;
+            if (vn < nloc && vn % PS_WCH == 0) {
                 windows(vn);
                 __syncthreads();
             }
-            if (tid == 0 && vn < nview && !*abort) {
+            if (tid == 0 && vn < nloc && !*abort) {
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 issue(vn);
                 last = vn;
             }
-        } else if ((v + 1) % PS_WCH == 0 && v + 1 < nview) {
+        } else if ((vi + 1) % PS_WCH == 0 && vi + 1 < nloc) {
             __syncthreads();
-            windows(v + 1);
+            windows(vi + 1);
             __syncthreads();
         }
     }
     if (!FALLBACK) {
         __syncthreads();
-        // every wait ended before this barrier, so all threads read the same
-        if (*abort) {
-            // the copies of the last PS_NS views issued may still be in flight
-            if (tid == 0)
-                for (int vp = max(last - (PS_NS - 1), 0); vp <= last; ++vp) {
-                    const int4 wv = window_of(vp);
-                    if (wv.x >= 0 && wv.z <= wv.w) mbar_wait_bounded(&bar[vp % PS_NS], (unsigned)((vp / PS_NS) & 1));
+        // every wait ended before this barrier, so all threads read the same;
+        // after one that gave up, the copies of the last PS_NS views issued
+        // may still be in flight
+        if (*abort && tid == 0)
+            for (int vp = max(last - (PS_NS - 1), 0); vp <= last; ++vp) {
+                const int4 wv = window_of(vp);
+                if (wv.x >= 0 && wv.z <= wv.w) mbar_wait_bounded(&bar[vp % PS_NS], (unsigned)((vp / PS_NS) & 1));
+            }
+        if (CS == 1) {
+            if (*abort) return;
+            if (tid == 0) unfit[cta] = s_unfit;
+        } else {
+            // all CTAs of the cluster meet here, aborted or not, and leave
+            // together: each stores R / CS of the tile's slices
+            namespace cg = cooperative_groups;
+            cg::cluster_group cluster = cg::this_cluster();
+            __syncthreads();  // the drained stages become the sums
+            float* sums = reinterpret_cast<float*>(stages);
+#pragma unroll
+            for (int i = 0; i < R; ++i) sums[i * (PS_T * PS_T) + tid] = acc[i];
+            cluster.sync();
+            int bad = 0, left = 0;
+            for (int r = 0; r < CS; ++r) {
+                bad |= *cluster.map_shared_rank(&s_abort, r);
+                left |= *cluster.map_shared_rank(&s_unfit, r);
+            }
+            if (!bad) {
+                if (rank == 0 && tid == 0) unfit[cta] = left;
+                for (int i = rank * (R / CS); i < (rank + 1) * (R / CS); ++i) {
+                    float sum = 0.0f;
+                    for (int r = 0; r < CS; ++r) sum += cluster.map_shared_rank(sums, r)[i * (PS_T * PS_T) + tid];
+                    const int j = j0 + i;
+                    if (active && j < g.D) st(vol + (((size_t)b * g.D + j) * g.H + iy) * g.W + ix, sum);
                 }
+            }
+            cluster.sync();  // the others may still read this CTA's sums
             return;
         }
-        if (tid == 0) unfit[cta] = s_unfit;
     }
     if (!active) return;
 #pragma unroll
