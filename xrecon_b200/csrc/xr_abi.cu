@@ -418,6 +418,14 @@ Layout layout(int dim3d, int op, const Geom& g, int nbatch, int nview, int dtype
             l.tab = o;    o = align256(o + bytes + 512);  // three arrays, 256-byte aligned each
             l.flags = o;  o = align256(o + V * nbatch * sizeof(int));
         }
+    } else if (!dim3d && nbatch == 1 && (op == OP_A || (op == OP_BT && g.type != GEO_ARC))) {
+        // line tables (B^T on the arc detector chains its angles, Bw^T weighs
+        // every pixel: both walk)
+        const size_t bytes = line_table_entries(g.W, g.H) * sizeof(double2);
+        if (bytes <= IL_GROUP_MAX) {
+            l.tab = o;    o = align256(o + bytes);
+            l.flags = o;  o = align256(o + (size_t)(g.W + g.H) * sizeof(int));
+        }
     } else if (!dim3d && op >= 0 && nbatch > 1 && nview > 0) {
         const int nb = interleave_nb(nbatch), groups = (nbatch + nb - 1) / nb;
         // images are kept twice (rows, flipped columns)
@@ -1040,6 +1048,19 @@ int run2d(int op, const Geom& g, const TI* in, void* out, int dto, const float* 
     // 2D does not read (8 + 8 bytes per column)
     vt.colQ = vt.colR = nullptr;
     if (op == OP_AT || op == OP_B || op == OP_BW) vt.colWR = reinterpret_cast<float4*>(ws + l.colQ);
+    if (l.tab && (op == OP_A || op == OP_BT)) {
+        const Geom2F f = make_geom2f(g);
+        const LineTable tab{reinterpret_cast<double2*>(ws + l.tab), reinterpret_cast<int*>(ws + l.flags), g.W, g.H};
+        const int nset = nview * ((g.Nu + 1 + 255) / 256);
+        linetab2d_kernel<TI><<<nset + nbatch * ((g.W + g.H + 7) / 8), 256, 0, st>>>(g, ang, nview, vt, nset, in, tab);
+        if (int rc = check_cuda("linetab2d")) return rc;
+        const int kb = (g.Nu + 63) / 64, LS = split2d((double)kb * nview * nbatch, std::min(g.W, g.H));
+        const dim3 grid((kb + 8 / LS - 1) / (8 / LS), nview, nbatch);
+        const float cw = column_width(g, 0);
+        if (op == OP_A) cell2t_kernel<TI, OP_A><<<grid, 256, 0, st>>>(f, vt, tab, in, out, dto, nview, cw, LS);
+        else cell2t_kernel<TI, OP_BT><<<grid, 256, 0, st>>>(f, vt, tab, in, out, dto, nview, cw, LS);
+        return check_cuda("cell2t");
+    }
     if (l.tab) {
         const float cw = column_width(g, 0);
         const Geom2F f = make_geom2f(g);
@@ -1333,7 +1354,7 @@ int helical(int op, const Geom& g, const HelOpts& o, const float* in, float* out
 
 struct RaggedLayout {
     size_t desc, sync;
-    std::vector<size_t> hdr, bA, bB, colWR, colE, colF, colM, arc, imgT, filt, tab, flags;
+    std::vector<size_t> hdr, bA, bB, colWR, colE, colF, colM, arc, lines, lflags, filt, tab, flags;
     size_t total;
 };
 
@@ -1358,10 +1379,9 @@ namespace xr {
 namespace {
 
 int ragged_tiles(const Geom& g, int nview, int list) {
-    const int hw = g.H * g.W;
-    if (list == 0) return nview + (hw + 1023) / 1024;
+    if (list == 0) return nview + (g.W + g.H + 7) / 8;
     if (list == 1) return nview;
-    if (list < 6) return nview * ((g.Nu + (32 << (list - 2)) - 1) / (32 << (list - 2)));
+    if (list < 6) return nview * ((g.Nu + (64 << (list - 2)) - 1) / (64 << (list - 2)));
     return pix2t_ctas(g.W, g.H, 1 << (list - 6));
 }
 
@@ -1756,7 +1776,8 @@ int xr_ragged2d_plan_create(const xr_ragged2d_instance* inst, int ninst, xr_ragg
         L.colM.push_back(o); o = align256(o + Vs * g.Nu * sizeof(float));
         L.arc.push_back(o);
         if (g.type == GEO_ARC) o = align256(o + 2 * Vs * (g.Nu + 1) * sizeof(float4));  // Bw's chained walks
-        L.imgT.push_back(o); o = align256(o + (size_t)g.H * g.W * sizeof(float));
+        L.lines.push_back(o); o = align256(o + line_table_entries(g.W, g.H) * sizeof(double2));
+        L.lflags.push_back(o); o = align256(o + (size_t)(g.W + g.H) * sizeof(int));
         L.filt.push_back(o); o = align256(o + Vs * g.Nu * sizeof(float));
         L.tab.push_back(o);  o = align256(o + Vs * (g.Nu + 2) * ROW_ENTRY_BYTES + 512);
         L.flags.push_back(o); o = align256(o + Vs * sizeof(int));
@@ -1814,7 +1835,7 @@ int xr_ragged2d_plan_bind(xr_ragged2d_plan* P, const float* images, float* sino,
         r.cw = column_width(r.g, 0);
         r.scale = in.scale;
         r.img = images + in.img_offset;
-        r.imgT = reinterpret_cast<float*>(ws + L.imgT[i]);
+        r.lines = LineTable{reinterpret_cast<double2*>(ws + L.lines[i]), reinterpret_cast<int*>(ws + L.lflags[i]), r.g.W, r.g.H};
         r.sino = sino + in.sino_offset;
         r.filt_out = reinterpret_cast<float*>(ws + L.filt[i]);
         r.tab = row_table_at(ws + L.tab[i], (size_t)in.nview * (r.g.Nu + 2));

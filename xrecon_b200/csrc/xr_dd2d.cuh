@@ -14,7 +14,8 @@
 //     weight is known;
 //   - a pixel-gather thread owns a 2 x 2 block of pixels, whose edges on a
 //     line are shared;
-//   - up to PT_MAX_BATCH images are gathered through per-view tables of the
+//   - single images are projected through tables of their lines' integrals
+//     (cell2t_kernel), and up to PT_MAX_BATCH images are gathered through per-view tables of the
 //     detector row's integral (pix2t_kernel: one table entry per pixel edge,
 //     no column loop); larger batches walk the columns once for NB images
 //     (pix2d_kernel).
@@ -285,6 +286,168 @@ cell2d_kernel(const Geom g, const Geom2F f, const ViewTables vt, const TI* __res
         const int b = b0 + blockIdx.z * NB + e;
         if (b < nbatch) st_dt(sino, dto, ((size_t)b * nview + v) * f.Nu + col, acc[e] * scale);
     }
+}
+
+// ------------------------------------------ cell gather through line tables
+//
+// With x in pixel p of line L, the line integrated up to x is S(x) = Q_p + v_p x,
+// Q_p = sum_{j < p} v_j - v_p p, so a cell's sum over the line is S(upper
+// boundary) - S(lower boundary): one 16-byte entry and one FP64 FMA per boundary
+// (shared by two neighbouring cells), whatever the number of pixels.  FP64
+// throughout, so nothing is lost against adding the overlaps; S is
+// continuous, so the pixel may be taken from the FP32 position (one off for
+// the few positions within its rounding of an integer, by at most that
+// rounding times the pixels' difference).  Lines of both orientations are
+// tabulated, entries -1 .. npix (the outer ones continue S as a constant); lines
+// holding a non-finite value are flagged and walked pixel by pixel.
+struct LineTable {
+    double2* q;  // H lines of W + 2, then W lines of H + 2
+    int* flags;  // H, then W
+    int W, H;
+    __host__ __device__ __forceinline__ size_t start(bool rows, int L) const {
+        return rows ? (size_t)L * (W + 2) : (size_t)H * (W + 2) + (size_t)L * (H + 2);
+    }
+};
+__host__ __device__ inline size_t line_table_entries(int W, int H) { return (size_t)H * (W + 2) + (size_t)W * (H + 2); }
+
+// One line's table, by one warp: line l < H is image row l, the others the
+// columns from the bottom up.
+template <typename T>
+__device__ __forceinline__ void build_line_table(const T* img, const LineTable& t, int l, int lane) {
+    const bool rows = l < t.H;
+    const int L = rows ? l : l - t.H, n = rows ? t.W : t.H;
+    double2* q = t.q + t.start(rows, L);
+    double carry = 0.0;
+    bool bad = false;
+    if (lane == 0) q[0] = make_double2(0.0, 0.0);
+    for (int base = 0; base <= n; base += 32) {
+        const int p = base + lane;
+        double v = 0.0;
+        if (p < n) {
+            const float x = ld(rows ? img + (size_t)L * t.W + p : img + (size_t)(t.H - 1 - p) * t.W + L);
+            if (isfinite(x)) v = (double)x;
+            else bad = true;
+        }
+        double s = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double u = __shfl_up_sync(0xffffffffu, s, o);
+            if (lane >= o) s += u;
+        }
+        if (p <= n) q[p + 1] = make_double2(carry + (s - v) - v * (double)p, v);
+        carry += __shfl_sync(0xffffffffu, s, 31);
+    }
+    bad = __any_sync(0xffffffffu, bad);
+    if (lane == 0) t.flags[l] = bad;
+}
+
+// Blocks [0, nset): view tables; the rest: eight lines each of an image's table.
+template <typename T>
+__global__ void __launch_bounds__(256)
+linetab2d_kernel(const Geom g, const float* __restrict__ ang, const int nview, const ViewTables vt, const int nset,
+                 const T* __restrict__ in, LineTable tab) {
+    if ((int)blockIdx.x < nset) {
+        const int bpv = (g.Nu + 1 + 255) / 256;
+        const int v = blockIdx.x / bpv, k = (blockIdx.x % bpv) * 256 + threadIdx.x;
+        if (v < nview && k <= g.Nu) setup_view_entry(g, 0, ang[v], v, k, vt, g.type == GEO_ARC);
+        return;
+    }
+    const int per = (g.W + g.H + 7) / 8, id = blockIdx.x - nset, b = id / per;
+    const int l = (id % per) * 8 + (threadIdx.x >> 5);
+    if (l >= g.W + g.H) return;
+    tab.q += b * line_table_entries(g.W, g.H);
+    tab.flags += (size_t)b * (g.W + g.H);
+    build_line_table(in + (size_t)b * g.W * g.H, tab, l, threadIdx.x & 31);
+}
+
+// Cells k and k + 1 (k + 1 < Nu or dropped by the caller) of view v over lines
+// l0, l0 + ls, ...; img is the image itself (flagged lines).
+template <int MODE, typename T>
+__device__ __forceinline__ void cell2t_walk(const Geom2F& f, const ViewTables& vt, const ViewHdr& h, const int v,
+                                            const int k, const float cw, const int l0, const int ls,
+                                            const LineTable& tab, const T* img, float (&acc)[2]) {
+    const int Nu = f.Nu, nlines = h.nlines, npix = h.npix;
+    const bool rows = h.use_x;
+    const size_t ob = (size_t)v * (Nu + 1);
+    double A[3], B[3];
+#pragma unroll
+    for (int e = 0; e < 3; ++e) {
+        const int kk = min(k + e, Nu);
+        A[e] = vt.bA[ob + kk];
+        B[e] = vt.bB[ob + kk];
+    }
+    const double q0 = h.q0, q1 = h.q1;
+    const float dpixf = (float)h.dpix;
+    const int* flags = tab.flags + (rows ? 0 : tab.H);
+    for (int L = l0; L < nlines; L += ls) {
+        const double dL = (double)L;
+        float lf = cw;
+        if (MODE == OP_A) lf = dpixf * rcp_fast((float)fma(q1, dL, q0));
+        if (flags[L]) {
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const double pk = fma(B[c], dL, A[c]), pk1 = fma(B[c + 1], dL, A[c + 1]);
+                const int pa = max((int)floor(pk), 0), pb = min((int)ceil(pk1) - 1, npix - 1);
+                for (int p = pa; p <= pb; ++p) {
+                    const float w = (float)(fmin((double)(p + 1), pk1) - fmax((double)p, pk)) * lf;
+                    acc[c] = fmaf(w, ld(rows ? img + (size_t)L * tab.W + p : img + (size_t)(tab.H - 1 - p) * tab.W + L), acc[c]);
+                }
+            }
+            continue;
+        }
+        const double2* q = tab.q + tab.start(rows, L);
+        double S[3];
+#pragma unroll
+        for (int e = 0; e < 3; ++e) {
+            const double pos = fma(B[e], dL, A[e]);
+            const float pf = fminf(fmaxf((float)pos, -1.0f), (float)npix);
+            const double2 t = q[XR_BOUND((__float_as_int(__fadd_rd(pf, 12582912.0f)) - 0x4B400000) + 1, 0, npix + 1)];
+            S[e] = fma(t.y, pos, t.x);
+        }
+        acc[0] = fmaf(lf, (float)(S[1] - S[0]), acc[0]);
+        acc[1] = fmaf(lf, (float)(S[2] - S[1]), acc[1]);
+    }
+    // a column whose boundaries are not in order on the lines (a ray past 90
+    // degrees from the axis) overlaps nothing
+    const double nl = (double)(nlines - 1);
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+        if (!(A[c + 1] > A[c]) || !(fma(B[c + 1], nl, A[c + 1]) > fma(B[c], nl, A[c]))) acc[c] = 0.0f;
+}
+
+// A CTA's 8 warps are 8 / LS blocks of 64 columns times LS line slices;
+// blockIdx.z is the image.
+template <typename TI, int MODE>
+__global__ void __launch_bounds__(256)
+cell2t_kernel(const Geom2F f, const ViewTables vt, LineTable tab, const TI* __restrict__ img, void* __restrict__ sino,
+              const int dto, const int nview, const float cw, const int LS) {
+    __shared__ float red[8][2][32];
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const int nblk = 8 / LS, slice = wp / nblk;
+    const int k = ((blockIdx.x * nblk + wp % nblk) * 32 + lane) * 2;
+    const int v = blockIdx.y, b = blockIdx.z;
+    const ViewHdr& h = vt.hdr[v];
+    tab.q += b * line_table_entries(f.W, f.H);
+    tab.flags += (size_t)b * (f.W + f.H);
+    float acc[2] = {0.0f, 0.0f};
+    if (k < f.Nu) cell2t_walk<MODE>(f, vt, h, v, k, cw, slice, LS, tab, img + (size_t)b * f.W * f.H, acc);
+    if (LS > 1) {
+        red[wp][0][lane] = acc[0];
+        red[wp][1][lane] = acc[1];
+        __syncthreads();
+        if (slice) return;
+        for (int s = 1; s < LS; ++s) {
+            acc[0] += red[s * nblk + wp][0][lane];
+            acc[1] += red[s * nblk + wp][1][lane];
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+        if (k + c < f.Nu) {
+            const float scale = MODE == OP_A ? vt.colE[(size_t)v * f.Nu + k + c] : 1.0f;
+            const int col = h.keep ? k + c : f.Nu - 1 - (k + c);
+            st_dt(sino, dto, ((size_t)b * nview + v) * f.Nu + col, acc[c] * scale);
+        }
 }
 
 // ----------------------------------------------------------- pixel gather
@@ -575,6 +738,7 @@ __device__ __forceinline__ bool build_row_table(const ViewTables& vt, const int 
     const double* bA = vt.bA + (size_t)v * (Nu + 1);
     const double* bB = vt.bB + (size_t)v * (Nu + 1);
     const float4* ea = vt.arc ? vt.arc + 2 * (size_t)v * (Nu + 1) : nullptr;
+    const double nl = (double)(vt.hdr[v].nlines - 1);
     double ca = 0.0, cb = 0.0;  // sums over the columns before this round
     bool bad = false;
     if (tid == 0) {
@@ -590,8 +754,13 @@ __device__ __forceinline__ bool build_row_table(const ViewTables& vt, const int 
             A = bA[j];
             B = bB[j];
             if (isfinite(y)) {
-                a = (double)y * (bA[j + 1] - A);
-                b = (double)y * (bB[j + 1] - B);
+                // (a column whose boundaries are not in order on the lines, a
+                // ray past 90 degrees from the axis, overlaps nothing)
+                const double dA = bA[j + 1] - A, dB = bB[j + 1] - B;
+                if (dA > 0.0 && fma(dB, nl, dA) > 0.0) {
+                    a = (double)y * dA;
+                    b = (double)y * dB;
+                }
             } else {
                 bad = true;
             }

@@ -652,7 +652,7 @@ hel_wbp_kernel(const Geom g, const GeomF gf, const ViewTables vt, const HelOpts 
                         const float nf = tr - 12582912.0f;
 #ifdef XR_DEBUG_BOUNDS
                         const long long t = XR_BOUND((long long)r0 + 1 + (__float_as_int(tr) - 0x4B400000), 0, Nv + 1);
-                        const float2 e = __ldg(reinterpret_cast<const float2*>(tvb) + (size_t)t * Nu + XR_BOUND(col, 0, Nu - 1));
+                        const float2 e = __ldg(reinterpret_cast<const float2*>(tvb) + (size_t)t * tab_pitch(Nu) + XR_BOUND(col, 0, Nu - 1));
 #else
                         const float2 e = __ldg(reinterpret_cast<const float2*>(
                             cb + (size_t)(unsigned)__float_as_int(tr) * Nu8));

@@ -7,10 +7,10 @@
 // very different cost share the GPU without idle SMs.  Phases are separated
 // by a grid barrier whose waits are bounded (a timeout sets the device error
 // word and ends the kernel):
-//   0  per-view DD tables of every instance (FP64) and the flipped transpose
-//      of every image (lines of y-axis views);
-//   1  projection A, cell-owned: a tile is CW columns of one view, the
-//      256 / CW threads of a column split its lines and reduce in shared
+//   0  per-view DD tables of every instance (FP64) and the line tables of
+//      every image (xr_dd2d.cuh);
+//   1  projection A, cell-owned: a tile is CW pairs of columns of one view, the
+//      256 / CW threads of a pair split its lines and reduce in shared
 //      memory;
 //   2  FBP pre-filter of every sinogram row: cosine weight x correlation with
 //      the instance's filter taps (the same arithmetic as fbp_filter_kernel),
@@ -41,7 +41,7 @@ struct RaggedDev {
     float cw;       // backprojection column width
     float scale;    // FBP scale
     const float* img;
-    float* imgT;
+    LineTable lines;
     float* sino;
     float* filt_out;
     RowTable tab;   // row tables of filt_out and their flags (xr_dd2d.cuh)
@@ -51,7 +51,7 @@ struct RaggedDev {
     const float* filt;
     const float* cosw;
     // first tile of this instance in each tile list: [0] tables and
-    // transposes, [1] filter rows, [2 + i] projection with CW = 32 << i,
+    // line tables, [1] filter rows, [2 + i] projection with CW = 32 << i,
     // [6 + i] backprojection with VS = 1 << i
     int t0[10];
 };
@@ -137,14 +137,8 @@ ragged2d_fbp_kernel(const RaggedDev* __restrict__ inst, const int ninst, const i
         if (lt < I.nview) {
             for (int k = tid; k <= g.Nu; k += blockDim.x) setup_view_entry(g, 0, I.ang[lt], lt, k, I.vt, g.type == GEO_ARC);
         } else {
-            const int base = (lt - I.nview) * 1024;
-            for (int e = tid; e < 1024; e += blockDim.x) {
-                const int idx = base + e;
-                if (idx < g.H * g.W) {
-                    const int y = idx / g.W, x = idx - y * g.W;
-                    I.imgT[(size_t)x * g.H + (g.H - 1 - y)] = I.img[idx];
-                }
-            }
+            const int l = (lt - I.nview) * 8 + (tid >> 5);
+            if (l < g.W + g.H) build_line_table(I.img, I.lines, l, tid & 31);
         }
     }
     if (!grid_barrier(bar, nb)) return;
@@ -155,27 +149,25 @@ ragged2d_fbp_kernel(const RaggedDev* __restrict__ inst, const int ninst, const i
         for (int t = next_tile(&ctr[1]); t < totals.y; t = next_tile(&ctr[1])) {
             const RaggedDev& I = inst[find_instance(inst, ninst, lists.y, t)];
             const Geom& g = I.g;
-            const int nbk = (g.Nu + CW - 1) / CW;
+            const int nbk = (g.Nu + 2 * CW - 1) / (2 * CW);
             const int lt = t - I.t0[lists.y];
             const int v = lt / nbk, kb = lt - v * nbk;
             const int c = tid % CW, s = tid / CW;
-            const int k = kb * CW + c;
+            const int k = 2 * (kb * CW + c);
             const ViewHdr& h = I.vt.hdr[v];
-            const float* img = h.use_x ? I.img : I.imgT;
-            const int npix = h.npix;
-            float acc = 0.0f;
-            if (k < g.Nu)
-                cell2d_walk<OP_A>(g, I.f, I.vt, h, v, k, 0.0f, s, LS,
-                                  [&](int L, int p, float w) { acc = fmaf(w, img[L * npix + p], acc); });
-            sm[tid] = acc;
+            float acc[2] = {0.0f, 0.0f};
+            if (k < g.Nu) cell2t_walk<OP_A>(I.f, I.vt, h, v, k, 0.0f, s, LS, I.lines, I.img, acc);
+            sm[tid] = acc[0];
+            sm[256 + tid] = acc[1];
             __syncthreads();
-            if (s == 0 && k < g.Nu) {
-                float sum = 0.0f;
-                for (int j = 0; j < LS; ++j) sum += sm[j * CW + c];
-                sum *= I.vt.colE[(size_t)v * g.Nu + k];
-                const int col = h.keep ? k : g.Nu - 1 - k;
-                I.sino[(size_t)v * g.Nu + col] = sum;
-            }
+            if (s == 0)
+                for (int e = 0; e < 2 && k + e < g.Nu; ++e) {
+                    float sum = 0.0f;
+                    for (int j = 0; j < LS; ++j) sum += sm[e * 256 + j * CW + c];
+                    sum *= I.vt.colE[(size_t)v * g.Nu + k + e];
+                    const int col = h.keep ? k + e : g.Nu - 1 - (k + e);
+                    I.sino[(size_t)v * g.Nu + col] = sum;
+                }
         }
     }
     if (!grid_barrier(bar, nb)) return;

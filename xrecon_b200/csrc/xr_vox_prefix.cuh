@@ -280,7 +280,7 @@ vox_prefix3d_kernel(const Geom g, const GeomF gf, const ViewTables vt, const flo
 #ifdef XR_DEBUG_BOUNDS
                 auto entry = [&](float tr) -> float2 {
                     const long long t = XR_BOUND((long long)r0 + 1 + (__float_as_int(tr) - 0x4B400000), 0, Nv + 1);
-                    return __ldg(reinterpret_cast<const float2*>(tvb) + (size_t)t * Nu + XR_BOUND(col, 0, Nu - 1));
+                    return __ldg(reinterpret_cast<const float2*>(tvb) + (size_t)t * tab_pitch(Nu) + XR_BOUND(col, 0, Nu - 1));
                 };
 #else
                 auto entry = [&](float tr) -> float2 {
