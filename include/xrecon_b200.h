@@ -324,6 +324,11 @@ void xr_ragged2d_plan_destroy(xr_ragged2d_plan* plan);
 int xr_ctpd_load(const char* const* paths, int nfiles, int rows, int cols, int col_stride, int row_stride,
                  int nthreads, float* sino, float* views, int* failed_file);
 
+/* x[0..n) *= factor * the mean wrapped angular step of angles[nview], in place
+ * on the stream (the FBP's last factor, projector.py:303-313); zero when there
+ * are fewer than two angles. */
+int xr_angle_step_scale(float* x, size_t n, const float* angles, int nview, float factor, void* stream);
+
 /* Number of CUDA kernels this library has launched in this process (all
  * devices and threads). */
 unsigned long long xr_launch_count(void);

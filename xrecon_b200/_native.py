@@ -68,6 +68,8 @@ def lib():
     L.xr_dd2d_noalloc.restype = c_int
     L.xr_dd2d_noalloc.argtypes = [c_int, ctypes.POINTER(Geom2d), c_void_p, c_int, c_void_p, c_int,
                                   c_void_p, c_int, c_int, c_void_p]
+    L.xr_angle_step_scale.restype = c_int
+    L.xr_angle_step_scale.argtypes = [c_void_p, c_size_t, c_void_p, c_int, c_float, c_void_p]
     L.xr_fbp_filter.restype = c_int
     L.xr_fbp_filter.argtypes = [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int,
                                 c_void_p, c_void_p, c_void_p, c_void_p]
@@ -280,6 +282,18 @@ def fbp_filter(sino: torch.Tensor, nview: int, rows_per_view: int, cosw: torch.T
     if rc != 0:
         _raise(rc, "xr_fbp_filter")
     return out
+
+
+def angle_step_scale_(x: torch.Tensor, angles: torch.Tensor, factor: float) -> torch.Tensor:
+    """``x *= factor * mean_angle_step(angles)`` in place (contiguous float32), one launch."""
+    dev = x.device
+    ang = _angles(angles, dev)
+    with torch.cuda.device(dev):
+        rc = lib().xr_angle_step_scale(x.data_ptr(), x.numel(), ang.data_ptr(), ang.numel(), factor,
+                                       torch.cuda.current_stream(dev).cuda_stream)
+    if rc != 0:
+        _raise(rc, "xr_angle_step_scale")
+    return x
 
 
 def system_matrix(dim: int, geom, angles: torch.Tensor, device) -> torch.Tensor:

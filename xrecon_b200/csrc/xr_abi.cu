@@ -1655,6 +1655,16 @@ int xr_dd2d_noalloc(int op, const xr_geom2d* geom, const void* in, int dtype_in,
                      (size_t)XR_NOALLOC_SCRATCH_BYTES, stream, 1.0f);
 }
 
+int xr_angle_step_scale(float* x, size_t n, const float* angles, int nview, float factor, void* stream) {
+    using namespace xr;
+    Trace tr("xr_angle_step_scale");
+    if (n == 0) return XR_OK;
+    if (!x || (!angles && nview > 0) || nview < 0) return fail(XR_ERR_INVALID_ARGUMENT, "bad angle step arguments");
+    const unsigned blocks = (unsigned)std::min<size_t>((n + 1023) / 1024, 148 * 8);
+    angle_step_scale_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(x, n, angles, nview, factor);
+    return check_cuda("angle_step_scale");
+}
+
 unsigned long long xr_launch_count(void) { return xr::g_launches.load(std::memory_order_relaxed); }
 
 int xr_rebin_parallel(const void* in, int dtype_in, float* out, int nbatch, int nview, int Nv, int Nu,

@@ -601,6 +601,42 @@ vox_gather3d_kernel(const Geom g, const GeomF gf, const ViewTables vt, const TI*
     }
 }
 
+// ---------------------------------------------------------- FBP angle step
+
+// x *= factor * mean wrapped angular step |((d + pi) mod 2 pi) - pi|
+// (projector.py:303-313) in place.  Every block forms the mean from the angles
+// itself (a few KB from L2), so the step costs one launch instead of the eight
+// elementwise and reduction launches it replaces (35 us of a 240 us 2D FBP).
+__global__ void __launch_bounds__(256)
+angle_step_scale_kernel(float* __restrict__ x, const size_t n, const float* __restrict__ ang, const int nview,
+                        const float factor) {
+    __shared__ double sums[8];
+    const float pi = 3.14159265358979323846f, two_pi = 6.28318530717958647692f;
+    double s = 0.0;
+    for (int i = threadIdx.x; i + 1 < nview; i += 256) {
+        float m = fmodf(__fadd_rn(__fsub_rn(ang[i + 1], ang[i]), pi), two_pi);
+        if (m < 0.0f) m = __fadd_rn(m, two_pi);
+        s += (double)fabsf(__fsub_rn(m, pi));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) sums[threadIdx.x >> 5] = s;
+    __syncthreads();
+    s = 0.0;
+    for (int w = 0; w < 8; ++w) s += sums[w];
+    const float scale = nview < 2 ? 0.0f : (float)(s / (double)(nview - 1)) * factor;
+    const size_t stride = (size_t)gridDim.x * 256;
+    size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
+    const bool vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+    const size_t n4 = vec ? n / 4 : 0;
+    for (; i < n4; i += stride) {
+        float4 v = reinterpret_cast<float4*>(x)[i];
+        v.x *= scale; v.y *= scale; v.z *= scale; v.w *= scale;
+        reinterpret_cast<float4*>(x)[i] = v;
+    }
+    for (i = 4 * n4 + (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += stride) x[i] *= scale;
+}
+
 // -------------------------------------------------------------- FBP filter
 
 // out[row, i] = sum_j x[row, j] * filt[j - i + Nu - 1], x = in * cosw * parker.

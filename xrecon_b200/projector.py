@@ -155,9 +155,7 @@ class _ProjectorBase(nn.Module):
                 redundant = False
         elif redundant is None:
             redundant = True
-        scale = self._mean_angle_step(angles.to(torch.float32))
-        if redundant:
-            scale = scale / 2
+        factor = 0.5 if redundant else 1.0
         Nu = self._num_u()
         wt = self.weight
         needs_grad = torch.is_grad_enabled() and (
@@ -166,6 +164,7 @@ class _ProjectorBase(nn.Module):
             pw_t = None if pw is None else pw.to(device=sino.device, dtype=torch.float32)
             filtered = _FilterRows.apply(sino.to(torch.float32), wt, filt, pw_t, angles.numel(), rows_per_view)
             recon = self.backprojection_weighted(filtered.contiguous(), angles)
+            scale = self._mean_angle_step(angles.to(torch.float32)) * factor
             return recon * scale.to(device=recon.device, dtype=recon.dtype)
         with torch.no_grad():
             s = sino if sino.is_contiguous() else sino.contiguous()
@@ -174,9 +173,8 @@ class _ProjectorBase(nn.Module):
                 cosw=wt.detach().reshape(-1), filt=filt.detach().reshape(-1),
                 parker=None if pw is None else pw.detach().reshape(angles.numel(), Nu))
             recon = self.backprojection_weighted(filtered, angles)
-            if sino.dtype != torch.float32:
-                recon = recon.to(sino.dtype)
-            return recon * scale.to(device=recon.device, dtype=recon.dtype)
+            _native.angle_step_scale_(recon, angles, factor)
+            return recon if sino.dtype == torch.float32 else recon.to(sino.dtype)
 
 
 class Projector2d(_ProjectorBase):
@@ -653,12 +651,12 @@ class HelicalProjector3d(nn.Module):
         wt = self.weight
         needs_grad = torch.is_grad_enabled() and (
             sino.requires_grad or (isinstance(filt, Tensor) and filt.requires_grad) or wt.requires_grad)
-        scale = mean_angle_step(angles)
         if needs_grad:
             sw = sino * wt.to(device=sino.device, dtype=sino.dtype)
             ones = torch.ones(Nu, device=sino.device, dtype=torch.float32)
             filtered = _FilterRows.apply(sw.to(torch.float32), ones, filt, None, V, Nv)
             recon = self.backprojection_weighted(filtered.contiguous(), angles, sp)
+            scale = mean_angle_step(angles)
             return recon * scale.to(device=recon.device, dtype=recon.dtype)
         with torch.no_grad():
             s = sino if sino.is_contiguous() else sino.contiguous()
@@ -668,7 +666,7 @@ class HelicalProjector3d(nn.Module):
                                           filt=filt.detach().reshape(-1),
                                           parker=wt.detach().reshape(Nv, Nu))
             recon = self.backprojection_weighted(filtered, angles, sp)
-            return recon * scale.to(device=recon.device, dtype=recon.dtype)
+            return _native.angle_step_scale_(recon, angles, 1.0)
 
     helical_fdk = filtered_backprojection
 
