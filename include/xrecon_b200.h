@@ -178,14 +178,17 @@ int xr_set_wait_limits(long long tma_polls, long long barrier_polls);
 int xr_test_hooks(unsigned int hooks);
 
 /* Staging plan of the 3D projection kernel for this geometry: whether the
- * TMA line windows are used, their box size (pixels x z voxels), and whether
- * the fine-row kernel (detector rows shorter than a voxel) is chosen. */
+ * TMA line windows are used, their box size (pixels x z voxels) at the default
+ * launch shape (eight warps of 8 or 16 rows; the launch may take another,
+ * planned the same way), and whether the fine-row kernel (detector rows shorter
+ * than a voxel) is chosen. */
 int xr_cell_plan(const xr_geom3d* geom, int* ok, int* box_pixels, int* box_z, int* rows_per_thread, int* fine);
 
 /* Staging plan of the 3D prefix backprojection (B, Bw, A^T) for this
  * geometry: whether each view's table footprint is staged into shared memory
- * (flat, parallel and arc detectors with an even column count), and the box
- * size in table columns x rows.  Host-only; no device is touched. */
+ * as it is (flat, parallel and arc detectors with an even column count; odd
+ * counts are staged through tables padded by a column and reported as not ok),
+ * and the box size in table columns x rows.  Host-only; no device is touched. */
 int xr_pfx_stage_plan(const xr_geom3d* geom, int* ok, int* box_cols, int* box_rows);
 
 /* Testing aid: nonzero routes every operator through the plain (non-TMA)
