@@ -24,7 +24,7 @@
 // Measured on a B200, before (one thread per output, no split, no tables) and
 // now, us: FBP of 256 x 256 pixels from 720 fan-flat views 1043 -> 219 (Bw 1006
 // -> 150); a batch of eight 512 x 512 arc slices, A + A^T over 360 views, 10825 ->
-// 1732; A + FBP of 16 ragged fan-arc instances 20344 -> 10730.  The pixel gathers
+// 1628; A + FBP of 16 ragged fan-arc instances 20344 -> 10730.  The pixel gathers
 // are held by the latency of their table entries in L1 and by conversions, the
 // batched walks by L1 wavefronts and lanes in different columns.
 #pragma once
@@ -652,8 +652,11 @@ __host__ __device__ inline int pix2d_tiles(int W, int H) {
 // A CTA's 8 warps are 8 / VS tiles times VS view slices.  NB = 1: the
 // sinograms [batch][view][column] of type TI; NB > 1: their interleaved FP32
 // copy.  blockIdx.y is the group of NB images.
+// A^T of eight images held at 80 registers (three CTAs per SM; 126 unbound, 24
+// bytes of spills): a batch of eight 512 x 512 slices, A + A^T, 1784 -> 1675 us; B
+// and Bw got slower that way (167 -> 190, 1235 -> 1266 us) and stay unbound.
 template <typename TI, int NB, int MODE>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, MODE == OP_AT && NB == 8 ? 3 : 1)
 pix2d_kernel(const Geom2F f, const ViewTables vt, const TI* __restrict__ sino, void* __restrict__ img,
              const int dto, const int nview, const int b0, const int nbatch, const float cw, const float oscale,
              const int VS) {
