@@ -23,7 +23,7 @@
 //
 // Measured on a B200, before (one thread per output, no split, no tables) and
 // now, us: FBP of 256 x 256 pixels from 720 fan-flat views 1043 -> 219 (Bw 1006
-// -> 150); a batch of eight 512 x 512 arc slices, A + A^T over 360 views, 10825 ->
+// -> about 180, the call less its other launches); a batch of eight 512 x 512 arc slices, A + A^T over 360 views, 10825 ->
 // 1628; A + FBP of 16 ragged fan-arc instances 20344 -> 10730.  The pixel gathers
 // are held by the latency of their table entries in L1 and by conversions, the
 // batched walks by L1 wavefronts and lanes in different columns.
