@@ -122,3 +122,27 @@ def test_fbp2d_trainable_filter_and_weight_gradients(cuda):
     (filtered * bwt * scale).sum().backward()
     assert rel_l2(P.filter.grad.cpu().numpy(), f.grad.numpy()) < 1e-5
     assert rel_l2(P.weight.grad.cpu().numpy(), w.grad.numpy()) < 1e-5
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("parker", [False, True])
+def test_fbp_of_16_bit_sinograms_scales_in_their_type(cuda, dtype, parker):
+    """A 16-bit result is the reconstruction rounded to its type times the angular step rounded to its type, bit for
+    bit, as ``recon * scale`` gives it (the reference's last line)."""
+    from xrecon_b200 import _native
+    from xrecon_b200.projector import mean_angle_step
+    for P, name in ((_projector2d("flat", "ramp"), "fbp2d_flat_parker"), (_projector3d("flat"), "fdk3d_flat")):
+        P = P.to(cuda)
+        g = load_golden(name)
+        if parker and "parker" not in g:
+            continue
+        sino = torch.from_numpy(g["sino"]).to(cuda, dtype)
+        ang = torch.from_numpy(g["angles"]).to(cuda)
+        got = P.filtered_backprojection(sino, ang, parker=parker)
+        pw = P.parker_weight(ang).reshape(ang.numel(), -1) if parker else None
+        rows = sino.shape[3] if sino.dim() == 5 else 1
+        filtered = _native.fbp_filter(sino, nview=ang.numel(), rows_per_view=rows, cosw=P.weight.detach().reshape(-1),
+                                      filt=P.filter.detach().reshape(-1), parker=pw)
+        recon = P.backprojection_weighted(filtered, ang).to(dtype)
+        scale = mean_angle_step(ang) * (1.0 if parker else 0.5)
+        assert got.dtype == dtype and torch.equal(got, recon * scale.to(dtype)), name

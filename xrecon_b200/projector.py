@@ -173,8 +173,12 @@ class _ProjectorBase(nn.Module):
                 cosw=wt.detach().reshape(-1), filt=filt.detach().reshape(-1),
                 parker=None if pw is None else pw.detach().reshape(angles.numel(), Nu))
             recon = self.backprojection_weighted(filtered, angles)
-            _native.angle_step_scale_(recon, angles, factor)
-            return recon if sino.dtype == torch.float32 else recon.to(sino.dtype)
+            if sino.dtype == torch.float32:
+                return _native.angle_step_scale_(recon, angles, factor)
+            # 16-bit results are rounded before the scale, which is of their type
+            scale = self._mean_angle_step(angles.to(torch.float32)) * factor
+            recon = recon.to(sino.dtype)
+            return recon * scale.to(device=recon.device, dtype=recon.dtype)
 
 
 class Projector2d(_ProjectorBase):
