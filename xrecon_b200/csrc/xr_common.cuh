@@ -413,11 +413,14 @@ __device__ __forceinline__ float guess_atan2f(float y, float x) {
 constexpr float XR_GUESS_ATAN_ERR = 4.0e-6f;  // bound used to widen brackets
 
 // The same with an eight-term polynomial fitted the same way (max error 1.2e-7
-// rad in FP32, its rounding), for callers that take the column as it is.
-__device__ __forceinline__ float fine_atan2f(float y, float x) {
+// rad in FP32, its rounding), for callers that take the column as it is except
+// near a boundary.
+// `inv` is 1 / max(|x|, |y|).
+__device__ __forceinline__ float fine_atan2f(float y, float x, float& inv) {
     const float ax = fabsf(x), ay = fabsf(y);
     const float mx = fmaxf(ax, ay), mn = fminf(ax, ay);
-    const float t = mx > 0.0f ? mn * rcp_fast(mx) : 0.0f;
+    inv = rcp_fast(mx);
+    const float t = mx > 0.0f ? mn * inv : 0.0f;
     const float t2 = t * t;
     float p = -0.0040545593947172165f;
     p = fmaf(p, t2, 0.021862929686903954f);

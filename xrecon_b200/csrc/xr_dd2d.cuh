@@ -29,6 +29,8 @@
 // batched walks by L1 wavefronts and lanes in different columns.
 #pragma once
 
+#include <cmath>
+
 #include <cooperative_groups.h>
 
 #include "xr_kernels.cuh"
@@ -45,6 +47,9 @@ struct Geom2F {
     float x0, y0, xc0, yc0;  // left / bottom image edge, centre of column 0 / row 0
     float dx, dy, inv_dx, inv_dy;
     float sod, shu, du, inv_du, half_nu;
+    // error bound of pix2t_view's FP32 column position, in columns: eps0 + eps1
+    // / distance from the source (flat: along the central ray), at most epsw
+    float eps0, eps1, epsw;
     int W, H, Nu, type;
 };
 
@@ -59,6 +64,29 @@ __host__ __device__ inline Geom2F make_geom2f(const Geom& g) {
     f.sod = (float)g.sod; f.shu = (float)g.shu; f.du = (float)g.du;
     f.inv_du = (float)(1.0 / g.du);
     f.half_nu = 0.5f * (float)g.Nu;
+    // First-order sums of the roundings, u = 2^-24 each.  r bounds |x| and |y| together (its square root of
+    // two is in the factors), U the detector's half-width.
+    const double u = std::ldexp(1.0, -24);
+    const double hx = 0.5 * g.W * g.dx + std::fabs(g.shx), hy = 0.5 * g.H * g.dy + std::fabs(g.shy);
+    const double r = std::sqrt(hx * hx + hy * hy), U = 0.5 * g.Nu * g.du + std::fabs(g.shu);
+    double e0 = u * 2.0 * g.Nu, e1 = 0.0, near = 1.0;
+    if (g.type == GEO_FLAT) {
+        // u = sod (x cos + y sin) / (sod + x sin - y cos)
+        e0 += u * 3.0 * U / g.du;
+        e1 = u * (4.3 * g.sod * r + U * (2.0 * g.sod + 4.3 * r)) / g.du;
+        near = g.sod - r;
+    } else if (g.type == GEO_ARC) {
+        // atan2 of the point seen from the source, and the float32 axis
+        // positions of the boundaries (arc_axis_f; within 1.7e-7 rad)
+        e0 += (u * 1.5 + 1.3e-7 + 1.7e-7) / g.du;
+        e1 = u * 1.5 * (r + g.sod) / g.du;
+        near = (g.sod - r) * 0.7;  // the larger component of a vector of that length
+    } else {
+        e0 += u * 4.3 * r / g.du;
+    }
+    f.eps0 = (float)e0;
+    f.eps1 = (float)e1;
+    f.epsw = (float)(e0 + e1 / near);
     f.W = g.W; f.H = g.H; f.Nu = g.Nu; f.type = g.type;
     return f;
 }
@@ -708,19 +736,20 @@ pix2d_kernel(const Geom2F f, const ViewTables vt, const TI* __restrict__ sino, v
 // A pixel's backprojection from the view is S(upper edge) - S(lower edge): one
 // table entry and two FP64 FMAs per edge, whatever the number of columns, with
 // no loop and no divergence.  Sums and differences are FP64, so the table
-// loses nothing against adding the overlaps one by one.  S is continuous, so
-// a column taken one off for an edge within the FP32 guess's error eps of its
-// boundary (about 1e-4 columns) changes S by at most eps of the columns'
-// difference, and only for a share eps of the edges.
+// loses nothing against adding the overlaps one by one.  The column of an edge
+// comes from an FP32 position; within that position's error bound of a boundary
+// (RowEps::e, about 1e-4 to 1e-3 columns) the FP64 boundary decides.
 //
 // On the arc detector B and Bw walk each pixel's columns with float32 angles
 // chained from its first column (ArcChain): boundary j inside the pixel lies
 // delta_j = (t_j - angle_j) dD/dangle_j off its direct position, which adds
 // delta_j (y_{j-1} - y_j) to the pixel; entry j carries angle_j and that
-// factor.
+// factor.  A pixel with an edge so close to a boundary that its column is uncertain,
+// or that the boundary may cross the edge by its offset, is walked (pixel_walk).
 //
 // A row holding an infinity or a NaN would spread it over every later entry;
-// such rows are flagged and walked column by column instead (pix2d_view).
+// such rows are walked column by column instead (pix2d_view), and so are views
+// whose column positions FP32 leaves uncertain by a quarter of a column.
 //
 // Entries -1 .. Nu of a row are at [0 .. Nu + 1], in three arrays (a lane's
 // neighbours then load neighbouring words): {QA, QB}, y, and on the arc
@@ -736,6 +765,26 @@ struct RowTable {
 };
 constexpr size_t ROW_ENTRY_BYTES = sizeof(double2) + sizeof(float) + sizeof(float2);
 constexpr int PT_MAX_BATCH = 4;
+
+// Of a row: error bound of its view's column positions without the distance
+// term (columns; ROW_WALK: the row is walked), and the rounding of a boundary
+// angle (columns; arc detector).
+struct RowEps {
+    float e, q;
+};
+constexpr float ROW_WALK = 2.0f;
+
+__device__ __forceinline__ RowEps row_eps(const Geom2F& f, const ViewHdr& h, bool bad) {
+    RowEps r{f.eps0, 0.0f};
+    if (f.type == GEO_ARC) {
+        // half a unit of the largest angle: 2^-24 of its power of two
+        const float a = fabsf((float)h.beta) + fabsf(f.shu) + f.half_nu * f.du;
+        r.q = __int_as_float((__float_as_int(fmaxf(a, 1.0e-6f)) & 0x7f800000) - (24 << 23)) * f.inv_du;
+        r.e += 1.1f * r.q;
+    }
+    if (bad || !(f.epsw + 1.1f * r.q < 0.25f)) r.e = ROW_WALK;
+    return r;
+}
 
 // The table of one detector row (the outer entries continue S as a
 // constant), by a whole CTA of 256 threads; val(j)
@@ -806,8 +855,8 @@ __device__ __forceinline__ bool build_row_table(const ViewTables& vt, const int 
 // View tables and row tables of one view per CTA, for all images of the batch.
 template <typename TI, bool SCALE>
 __global__ void __launch_bounds__(256)
-table2d_kernel(const Geom g, const float* __restrict__ ang, const int nview, const ViewTables vt,
-               const TI* __restrict__ sino, const int nbatch, const RowTable tab, int* __restrict__ flags) {
+table2d_kernel(const Geom g, const Geom2F f, const float* __restrict__ ang, const int nview, const ViewTables vt,
+               const TI* __restrict__ sino, const int nbatch, const RowTable tab, RowEps* __restrict__ eps) {
     __shared__ double2 sums[8];
     const int v = blockIdx.x, Nu = g.Nu;
     for (int k = threadIdx.x; k <= Nu; k += 256) setup_view_entry(g, 0, ang[v], v, k, vt, g.type == GEO_ARC);
@@ -820,7 +869,7 @@ table2d_kernel(const Geom g, const float* __restrict__ ang, const int nview, con
             const float x = ld(y + (keep ? j : Nu - 1 - j));
             return SCALE ? x * vt.colE[(size_t)v * Nu + j] : x;
         });
-        if (threadIdx.x == 0) flags[row] = bad;
+        if (threadIdx.x == 0) eps[row] = row_eps(f, vt.hdr[v], bad);
     }
 }
 
@@ -833,17 +882,52 @@ __device__ __noinline__ float4 pix2d_view_walk(const Geom2F& f, const ViewTables
     return make_float4(acc[0][0][0], acc[0][1][0], acc[1][0][0], acc[1][1][0]);
 }
 
+// View v's contribution to pixel (ix, iy) on the arc detector (B, Bw), its columns
+// walked with chained angles as pix2d_axis walks them but with every direct
+// boundary in FP64; y is the row's values, entry j + 1 that of column j.
+template <int MODE>
+__device__ __noinline__ float pixel_walk(const Geom2F& f, const ViewTables& vt, int v, int ix, int iy, float cw,
+                                         const float* y) {
+    const ViewHdr& h = vt.hdr[v];
+    const int Nu = f.Nu, keep = h.keep, p = h.use_x ? ix : f.H - 1 - iy;
+    const size_t ob = (size_t)v * (Nu + 1);
+    const double dL = (double)(h.use_x ? iy : ix), dp = (double)p;
+    auto pos = [&](int b) { return fma(vt.bB[ob + b], dL, vt.bA[ob + b]); };
+    const float px = fmaf((float)ix, f.dx, f.xc0), py = fmaf(-(float)iy, f.dy, f.yc0);
+    const float rx = px - h.sxr, ry = py - h.syr;
+    const float u = guess_atan2f(h.dcx * ry - h.dcy * rx, h.dcx * rx + h.dcy * ry) * f.inv_du;
+    int k = (int)fminf(fmaxf(f.half_nu + (keep ? u : -u), 0.0f), (float)(Nu - 1));
+    while (k > 0 && pos(k) > dp) --k;
+    while (k < Nu - 1 && pos(k + 1) <= dp) ++k;
+    const float q = (float)fma(h.q1, dL, h.q0), qd = q * (h.use_x ? f.inv_dx : f.inv_dy);  // pixels per axis unit
+    const float4* ea = vt.arc + 2 * ob;
+    float s = 0.0f, lo = fmaxf(0.0f, (float)(pos(k) - dp));
+    ArcChain ch;
+    ch.start(ea, k, keep, f.du);
+    for (; k < Nu && lo < 1.0f; ++k) {
+        float d = ch.next_linear(ea, k + 1);
+        if (k + 1 == Nu) d = fminf(d, 0.0f);  // the detector's end
+        const float hi = fmaf(d, qd, (float)(pos(k + 1) - dp)), c = fminf(1.0f, hi) - lo;
+        if (c > 0.0f) s = fmaf(c, y[k + 1], s);
+        lo = fmaxf(lo, hi);
+    }
+    return s * (MODE == OP_BW ? cw * fbp_weight2d(f, h.sxr, h.syr, px, py) : cw);
+}
+
 // View v's contribution to a P2 x P2 block through its row table.  Both axes
 // run the same code (line j, pixel i of its run), the sums are placed at the
-// end.
-template <int MODE>
-__device__ __forceinline__ void pix2t_view(const Geom2F& f, const ViewTables& vt, const int v, const int ix0,
-                                           const int iy0, const float cw, const RowTable tab, float (&acc)[P2][P2]) {
+// end.  CHAIN: chained boundary angles (B and Bw on the arc detector); returns the
+// pixels left out (bit row P2 + column), which the caller walks: those with an edge
+// within its position's error bound of a boundary, and those whose chained offsets
+// may cross an edge.
+template <int MODE, bool CHAIN>
+__device__ __forceinline__ unsigned pix2t_view(const Geom2F& f, const ViewTables& vt, const int v, const int ix0,
+                                           const int iy0, const float cw, const RowTable tab, const RowEps eps,
+                                           float (&acc)[P2][P2]) {
     const ViewHdr* h = vt.hdr + v;
     const int4 hi = *reinterpret_cast<const int4*>(&h->use_x);
     const float4 hs = *reinterpret_cast<const float4*>(&h->sf);  // sin, cos, source
     const bool use_x = hi.x != 0, keep = hi.y != 0;
-    const bool chain = MODE != OP_AT && vt.arc;
     const int Nu = f.Nu;
     const int p0 = use_x ? ix0 : f.H - P2 - iy0, L0 = use_x ? iy0 : ix0;  // first pixel of the runs, first line
     // the runs' first edge, the step along a run and from line to line
@@ -855,32 +939,54 @@ __device__ __forceinline__ void pix2t_view(const Geom2F& f, const ViewTables& vt
     const float sg = keep ? f.inv_du : -f.inv_du;
     const float k0f = f.half_nu - (f.type == GEO_ARC ? 0.0f : f.shu * sg);
     float t[P2][P2];
+    unsigned walk = 0;  // pixels to walk, bit j P2 + i
 #pragma unroll
     for (int j = 0; j < P2; ++j) {
         const double dL = (double)(L0 + j);
         const float xa = fmaf((float)j, lx, x0), ya = fmaf((float)j, ly, y0);
         double S[P2 + 1];
         int ki[P2 + 1];  // entry of each edge's column (0: before the first)
+        float off[P2 + 1], em = 0.0f;  // distance of each edge from its column's middle, the edges' error bound
 #pragma unroll
         for (int i = 0; i <= P2; ++i) {
             const float x = fmaf((float)i, ex, xa), y = fmaf((float)i, ey, ya);
-            float u;
+            float u, inv = 0.0f;
             if (f.type == GEO_FLAT) {
-                u = f.sod * (x * hs.y + y * hs.x) * rcp_fast(f.sod + x * hs.x - y * hs.y);
+                inv = rcp_fast(f.sod + x * hs.x - y * hs.y);
+                u = f.sod * (x * hs.y + y * hs.x) * inv;
             } else if (f.type == GEO_ARC) {
                 const float rx = x - hs.z, ry = y - hs.w;
-                u = fine_atan2f(h->dcx * ry - h->dcy * rx, h->dcx * rx + h->dcy * ry);
+                u = fine_atan2f(h->dcx * ry - h->dcy * rx, h->dcx * rx + h->dcy * ry, inv);
             } else {
                 u = x * hs.y + y * hs.x;
             }
-            const float kf = fminf(fmaxf(fmaf(u, sg, k0f), -1.0f), (float)Nu);
+            // (half a column outside the detector is as good as any place there)
+            const float kf = fminf(fmaxf(fmaf(u, sg, k0f), -0.5f), (float)Nu + 0.5f);
             // floor by an add of 1.5 * 2^23 rounded down: the column in the low bits
-            ki[i] = XR_BOUND((__float_as_int(__fadd_rd(kf, 12582912.0f)) - 0x4B400000) + 1, 0, Nu + 1);
+            const float tr = __fadd_rd(kf, 12582912.0f);
+            ki[i] = XR_BOUND((__float_as_int(tr) - 0x4B400000) + 1, 0, Nu + 1);
+            off[i] = (kf - (tr - 12582912.0f)) - 0.5f;
+            em = fmaxf(em, fmaf(f.eps1, inv, eps.e));
+        }
+        bool near = false;
+#pragma unroll
+        for (int i = 0; i <= P2; ++i) near = near || fabsf(off[i]) > 0.5f - em;
+        if (!CHAIN && near) {
+#pragma unroll
+            for (int i = 0; i <= P2; ++i)
+                if (fabsf(off[i]) > 0.5f - em) {  // boundary b decides
+                    const int b = XR_BOUND(ki[i] - 1 + (off[i] > 0.0f), 0, Nu);
+                    const size_t ob = (size_t)v * (Nu + 1) + b;
+                    ki[i] = b + (fma(vt.bB[ob], dL, vt.bA[ob]) <= (double)(p0 + i));
+                }
+        }
+#pragma unroll
+        for (int i = 0; i <= P2; ++i) {
             const double2 q = tab.q[ki[i]];
             S[i] = fma((double)tab.y[ki[i]], (double)(p0 + i), fma(q.y, dL, q.x));
         }
         float lf = 1.0f;
-        if (MODE == OP_AT || chain) {
+        if (MODE == OP_AT || CHAIN) {
             const float q = (float)fma(h->q1, dL, h->q0);
             lf = MODE == OP_AT ? (use_x ? f.dx : f.dy) * rcp_fast(q) : q * (use_x ? f.inv_dx : f.inv_dy);
         }
@@ -888,11 +994,16 @@ __device__ __forceinline__ void pix2t_view(const Geom2F& f, const ViewTables& vt
         for (int i = 0; i < P2; ++i) {
             float s = (float)(S[i + 1] - S[i]);
             if (MODE == OP_AT) s *= lf;
-            if (chain && ki[i + 1] > ki[i]) {
+            if (CHAIN) {
                 // boundaries ka + 1 .. kb (entries ka + 2 ..) lie in the pixel;
-                // the walk starts at column ka
+                // the walk starts at column ka.  A boundary's offset is up to
+                // steps + 3 roundings.
+                const float ec = fmaf((float)(ki[i + 1] - ki[i] + 3), eps.q, em);
                 const int ka = max(ki[i] - 1, 0), kb = min(ki[i + 1] - 1, Nu);
-                if (kb > ka) {
+                if (off[i] < em - 0.5f || off[i] > 0.5f - ec || fabsf(off[i + 1]) > 0.5f - ec) {
+                    s = 0.0f;
+                    walk |= 1u << (use_x ? j * P2 + i : (P2 - 1 - i) * P2 + j);
+                } else if (kb > ka) {
                     const float step = keep ? f.du : -f.du;
                     float a = keep ? tab.c[ka + 1].x : __fadd_rn(tab.c[ka + 2].x, f.du), corr = 0.0f;
                     for (int b = ka + 1; b <= kb; ++b) {
@@ -926,6 +1037,45 @@ __device__ __forceinline__ void pix2t_view(const Geom2F& f, const ViewTables& vt
             }
             acc[r][c] = MODE == OP_AT ? acc[r][c] + s : fmaf(w, s, acc[r][c]);
         }
+    return walk;
+}
+
+// Views v0, v0 + vs, ... < nview of one block: row v's table and error bound at
+// tab.at(v) and eps[v], its values as src(v) gives them.  The few pixels that a
+// view leaves out are listed and walked together, every lane its own (walked at
+// once, a warp would wait for one of them in most views of an arc scan: a ragged
+// batch of 16 arc scans 14488 -> 12028 us).
+template <int MODE, bool CHAIN, typename Src>
+__device__ __forceinline__ void pix2t_views(const Geom2F& f, const ViewTables& vt, const RowTable tab, const RowEps* eps,
+                                            const int ix0, const int iy0, const float cw, const int v0, const int nview,
+                                            const int vs, Src&& src, float (&acc)[P2][P2]) {
+    constexpr int CAP = 16;
+    unsigned list[CAP];
+    int n = 0;
+    auto flush = [&]() {
+        for (int i = 0; i < n; ++i) {
+            const int v = list[i] >> 2, r = (list[i] >> 1) & 1, c = list[i] & 1;
+            const float s = pixel_walk<MODE>(f, vt, v, ix0 + c, iy0 + r, cw, tab.at(v, f.Nu).y);
+#pragma unroll
+            for (int e = 0; e < P2 * P2; ++e)
+                if (e == (int)(list[i] & 3)) acc[e / P2][e % P2] += s;
+        }
+        n = 0;
+    };
+    for (int v = v0; v < nview; v += vs) {
+        const RowEps e = eps[v];
+        if (e.e >= 1.0f) {
+            const float4 s = pix2d_view_walk<MODE>(f, vt, v, ix0, iy0, cw, src(v));
+            acc[0][0] += s.x; acc[0][1] += s.y; acc[1][0] += s.z; acc[1][1] += s.w;
+            continue;
+        }
+        const unsigned left = pix2t_view<MODE, CHAIN>(f, vt, v, ix0, iy0, cw, tab.at(v, f.Nu), e, acc);
+        if (CHAIN) {
+            for (unsigned m = left; m; m &= m - 1) list[n++] = (unsigned)v << 2 | (unsigned)(__ffs(m) - 1);
+            if (__any_sync(__activemask(), n > CAP - P2 * P2)) flush();
+        }
+    }
+    if (CHAIN) flush();
 }
 
 // Tiles of a CTA: 2 x 4 warp tiles when its 8 warps share the views, else 8 /
@@ -948,10 +1098,10 @@ __device__ __forceinline__ void pix2t_origin(const Geom2F& f, int VS, int cta, i
 // Warps of one CTA that share a view (VS = 1) also share its header and table
 // in L1; the cluster's sums meet through distributed shared memory, in rank
 // order.  blockIdx.y is the image.
-template <typename TI, int MODE>
+template <typename TI, int MODE, bool CHAIN>
 __global__ void __launch_bounds__(256, 4)
 pix2t_kernel(const __grid_constant__ Geom2F f, const __grid_constant__ ViewTables vt, const RowTable tab,
-             const int* __restrict__ flags, const TI* __restrict__ sino, void* __restrict__ img, const int dto,
+             const RowEps* __restrict__ eps, const TI* __restrict__ sino, void* __restrict__ img, const int dto,
              const int nview, const float cw, const float oscale, const int VS) {
     namespace cg = cooperative_groups;
     __shared__ float red[8][P2 * P2][32];
@@ -964,15 +1114,8 @@ pix2t_kernel(const __grid_constant__ Geom2F f, const __grid_constant__ ViewTable
     const size_t row0 = (size_t)blockIdx.y * nview;
     float acc[P2][P2] = {};
     if (ix0 < f.W && iy0 < f.H)
-        for (int v = slice; v < nview; v += VS * CS) {
-            if (flags[row0 + v]) {
-                const float4 s = pix2d_view_walk<MODE>(f, vt, v, ix0, iy0, cw,
-                                                       SinoLanes<TI, 1>{sino + (row0 + v) * f.Nu, 0});
-                acc[0][0] += s.x; acc[0][1] += s.y; acc[1][0] += s.z; acc[1][1] += s.w;
-            } else {
-                pix2t_view<MODE>(f, vt, v, ix0, iy0, cw, tab.at(row0 + v, f.Nu), acc);
-            }
-        }
+        pix2t_views<MODE, CHAIN>(f, vt, tab.at(row0, f.Nu), eps + row0, ix0, iy0, cw, slice, nview, VS * CS,
+                                 [&](int v) { return SinoLanes<TI, 1>{sino + (row0 + v) * f.Nu, 0}; }, acc);
     float* a = &acc[0][0];
     auto store = [&](int wt, const float* sum) {
         int x0, y0;

@@ -44,8 +44,8 @@ struct RaggedDev {
     LineTable lines;
     float* sino;
     float* filt_out;
-    RowTable tab;   // row tables of filt_out and their flags (xr_dd2d.cuh)
-    int* flags;
+    RowTable tab;   // row tables of filt_out and their error bounds (xr_dd2d.cuh)
+    RowEps* eps;
     float* recon;
     const float* ang;
     const float* filt;
@@ -199,7 +199,7 @@ ragged2d_fbp_kernel(const RaggedDev* __restrict__ inst, const int ninst, const i
         const int keep = I.vt.hdr[v].keep;
         const bool bad = build_row_table(I.vt, v, Nu, I.tab.at(v, Nu), row_sums,
                                          [&](int j) -> float { return y[keep ? j : Nu - 1 - j]; });
-        if (tid == 0) I.flags[v] = bad;
+        if (tid == 0) I.eps[v] = row_eps(I.f, I.vt.hdr[v], bad);
     }
     if (!grid_barrier(bar, nb)) return;
 
@@ -213,16 +213,9 @@ ragged2d_fbp_kernel(const RaggedDev* __restrict__ inst, const int ninst, const i
             pix2t_origin(I.f, VS, t - I.t0[lists.w], wp % ntile, lane, ix0, iy0);
             const bool active = ix0 < W && iy0 < H;
             float acc[P2][P2] = {};
-            if (active)
-                for (int v = slice; v < I.nview; v += VS) {
-                    if (I.flags[v]) {
-                        const float4 s = pix2d_view_walk<OP_BW>(I.f, I.vt, v, ix0, iy0, I.cw,
-                                                                FiltLanes{I.filt_out + (size_t)v * I.f.Nu});
-                        acc[0][0] += s.x; acc[0][1] += s.y; acc[1][0] += s.z; acc[1][1] += s.w;
-                    } else {
-                        pix2t_view<OP_BW>(I.f, I.vt, v, ix0, iy0, I.cw, I.tab.at(v, I.f.Nu), acc);
-                    }
-                }
+            auto row = [&](int v) { return FiltLanes{I.filt_out + (size_t)v * I.f.Nu}; };
+            if (active && I.vt.arc) pix2t_views<OP_BW, true>(I.f, I.vt, I.tab, I.eps, ix0, iy0, I.cw, slice, I.nview, VS, row, acc);
+            else if (active) pix2t_views<OP_BW, false>(I.f, I.vt, I.tab, I.eps, ix0, iy0, I.cw, slice, I.nview, VS, row, acc);
             float* a = &acc[0][0];
 #pragma unroll
             for (int e = 0; e < P2 * P2; ++e) sm[e * 256 + tid] = a[e];
