@@ -46,3 +46,93 @@ def test_every_edge_finds_its_column(cuda, scan, W, Nu, du, V):
         walked = rel_l2(_run(op, sino, opts, ang, cuda).cpu().numpy(), want)
         tabled = [rel_l2(_run(op, sino[i:i + 1], opts, ang, cuda).cpu().numpy(), want[i:i + 1]) for i in range(3)]
         assert max(tabled) < max(4e-7, 1.5 * walked), (op, tabled, walked)
+
+
+OUTLIERS = [1e20, float(np.finfo(np.float32).min), np.inf, np.nan]
+
+
+def _untouched(op, x, at, opts, ang):
+    """Oracle of x without the element `at` of every image, and the outputs that this element does not reach."""
+    alone, rest = np.zeros_like(x), x.copy()
+    alone[(slice(None), 0) + at] = 1.0
+    rest[(slice(None), 0) + at] = 0.0
+    return O.dd2d(op, rest, opts, ang), O.dd2d(op, alone, opts, ang) == 0
+
+
+@pytest.mark.parametrize("B", [1, 4, 8])
+@pytest.mark.parametrize("scan", ["parallel", "flat", "arc"])
+@pytest.mark.parametrize("value", OUTLIERS)
+def test_an_outlier_reaches_only_what_it_touches(cuda, scan, value, B):
+    """One very large, infinite or NaN pixel or cell: outputs that do not overlap it are those of the rest (1e-5
+    relative L2, the bound of every operator), and those that do carry it."""
+    opts = _opts(scan, 40, 31, 60, 1.6)
+    rng = np.random.default_rng(3)
+    ang = (np.arange(9) * 0.71 + 0.05).astype(np.float32)
+    img = rng.random((B, 1, 31, 40)).astype(np.float32)
+    sino = rng.random((B, 1, 9, 60)).astype(np.float32)
+    for op in OPS:
+        x, at = (img, (11, 9)) if op in IMAGE_IN else (sino, (4, 22))
+        want, free = _untouched(op, x, at, opts, ang)
+        x = x.copy()
+        x[(slice(None), 0) + at] = value
+        got = _run(op, x, opts, ang, cuda).cpu().numpy()
+        assert 0 < free.sum() < free.size
+        assert rel_l2(got[free], want[free]) < 1e-5, op
+        hit = np.abs(got[~free])
+        assert (hit > 1e12).any() if np.isfinite(value) else not np.isfinite(hit).all(), op
+
+
+@pytest.mark.parametrize("value", OUTLIERS)
+def test_an_outlier_in_a_ragged_batch(cuda, value):
+    """The same for the projections of a ragged batch; its filter spreads the value over every column of a view, so
+    of the reconstructions only the other instance's is compared."""
+    from xrecon_b200 import geometry as G
+    from xrecon_b200.projector import Projector2d
+    from xrecon_b200.ragged import RaggedFBP2d
+    P = [Projector2d(G.Volume2d((n, n - 3), 1.0), G.FanBeam2d(G.Detector2d(m, 2.2), 500.0, 1000.0, "arc")).to(cuda)
+         for n, m in ((40, 60), (33, 47))]
+    ang = [torch.arange(V) * (2 * math.pi / V) + 0.05 for V in (9, 14)]
+    rng = np.random.default_rng(4)
+    img = [rng.random((1, 1, n - 3, n)).astype(np.float32) for n in (40, 33)]
+    plan = RaggedFBP2d(P, ang)
+    clean = [r.clone() for r in plan([torch.from_numpy(x).to(cuda) for x in img])[1]]
+    opts = P[0].options.cpu().numpy()
+    want, free = _untouched("A", img[0], (11, 9), opts, ang[0].numpy())
+    img[0][0, 0, 11, 9] = value
+    sino, recon = plan([torch.from_numpy(x).to(cuda) for x in img])
+    got = sino[0].cpu().numpy()
+    assert 0 < free.sum() < free.size
+    assert rel_l2(got[free], want[free]) < 1e-5
+    assert torch.equal(recon[1], clean[1])
+
+
+@pytest.mark.parametrize("value", [1e20, np.inf])
+def test_an_outlier_in_a_ragged_row(cuda, value):
+    """Row tables of a ragged batch: with a filter of one tap the filtered row is the row itself, and a view that
+    holds the value is walked."""
+    from xrecon_b200 import geometry as G
+    from xrecon_b200.projector import Projector2d
+    from xrecon_b200.ragged import RaggedFBP2d
+    P = Projector2d(G.Volume2d((40, 37), 1.0), G.FanBeam2d(G.Detector2d(60, 2.2), 500.0, 1000.0, "arc")).to(cuda)
+    with torch.no_grad():
+        taps = torch.zeros_like(P.filter).reshape(-1)
+        taps[taps.numel() // 2] = 1.0
+        P.filter.copy_(taps.reshape(P.filter.shape))
+    ang = torch.arange(9) * 0.71 + 0.05
+    plan = RaggedFBP2d([P], [ang], graph=False)
+    img = torch.rand(37, 40, generator=torch.Generator().manual_seed(5)).to(cuda)
+    plan([img])
+    sino = plan.sino.clone().view(1, 1, 9, 60)
+    opts, w = P.options.cpu().numpy(), P.weight.detach().cpu().numpy().reshape(-1)
+    weighted = sino.cpu().numpy() * w
+    want, free = _untouched("BW", weighted, (4, 22), opts, ang.numpy())
+    plan.sino.view(9, 60)[4, 22] = value
+    plan.launch(project=False)
+    got = plan.reconstructions()[0].cpu().numpy()
+    d = ang.diff().double()
+    scale = float(((d + math.pi) % (2 * math.pi) - math.pi).abs().mean()) / 2
+    assert 0 < free.sum() < free.size
+    if np.isfinite(value):  # an infinity times the filter's zeros is NaN in every column of its view
+        assert rel_l2(got[free], want[free] * scale) < 1e-5
+    else:
+        assert not np.isfinite(got[~free]).any()

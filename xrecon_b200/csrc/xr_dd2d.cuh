@@ -328,13 +328,39 @@ cell2d_kernel(const Geom g, const Geom2F f, const ViewTables vt, const TI* __res
 // With x in pixel p of line L, the line integrated up to x is S(x) = Q_p + v_p x,
 // Q_p = sum_{j < p} v_j - v_p p, so a cell's sum over the line is S(upper
 // boundary) - S(lower boundary): one 16-byte entry and one FP64 FMA per boundary
-// (shared by two neighbouring cells), whatever the number of pixels.  FP64
-// throughout, so nothing is lost against adding the overlaps; S is
-// continuous, so the pixel may be taken from the FP32 position (one off for
-// the few positions within its rounding of an integer, by at most that
-// rounding times the pixels' difference).  Lines of both orientations are
-// tabulated, entries -1 .. npix (the outer ones continue S as a constant); lines
-// holding a non-finite value are flagged and walked pixel by pixel.
+// (shared by two neighbouring cells), whatever the number of pixels.  S is FP64,
+// of up to n |v|max in magnitude (n pixels), so a difference is off by a few
+// 2^-53 n |v|max: less than FP32 loses on pixels near the largest, but all of a
+// pixel that is 2^-40 of it.  Lines whose smallest value would lose 2^-18 of itself
+// (Spread::too_wide: one dead pixel of 1e20, a mask of the lowest float), and those
+// holding an infinity or a NaN, are flagged and walked pixel by pixel.  S is
+// continuous, so the pixel may be taken from the FP32 position (one off for the
+// few positions within its rounding of an integer, by at most that rounding times
+// the pixels' difference).  Lines of both orientations are tabulated, entries -1 ..
+// npix (the outer ones continue S as a constant).
+
+// Magnitudes of a table's values, as the bits of |v|: the largest (an infinity or
+// a NaN is above every finite one) and the smallest but zero.
+struct Spread {
+    unsigned most = 0u, least = 0xffffffffu;
+    __device__ __forceinline__ void add(float v) {
+        const unsigned b = (unsigned)__float_as_int(v) & 0x7fffffffu;
+        most = max(most, b);
+        if (b) least = min(least, b);
+    }
+    __device__ __forceinline__ void warp() {
+        most = __reduce_max_sync(0xffffffffu, most);
+        least = __reduce_min_sync(0xffffffffu, least);
+    }
+    // whether sums over positions of up to `reach` pixels are no good for these
+    // values: 2^-53 reach |v|max, a few times, is to stay below 2^-18 |v|min
+    __device__ __forceinline__ bool too_wide(float reach) const {
+        if (most == 0u) return false;
+        return most >= 0x7f800000u || !((double)__int_as_float((int)most) * (double)reach <=
+                                        8589934592.0 * (double)__int_as_float((int)least));
+    }
+};
+
 struct LineTable {
     double2* q;  // H lines of W + 2, then W lines of H + 2
     int* flags;  // H, then W
@@ -353,15 +379,15 @@ __device__ __forceinline__ void build_line_table(const T* img, const LineTable& 
     const int L = rows ? l : l - t.H, n = rows ? t.W : t.H;
     double2* q = t.q + t.start(rows, L);
     double carry = 0.0;
-    bool bad = false;
+    Spread spread;
     if (lane == 0) q[0] = make_double2(0.0, 0.0);
     for (int base = 0; base <= n; base += 32) {
         const int p = base + lane;
         double v = 0.0;
         if (p < n) {
             const float x = ld(rows ? img + (size_t)L * t.W + p : img + (size_t)(t.H - 1 - p) * t.W + L);
+            spread.add(x);
             if (isfinite(x)) v = (double)x;
-            else bad = true;
         }
         double s = v;
 #pragma unroll
@@ -372,8 +398,8 @@ __device__ __forceinline__ void build_line_table(const T* img, const LineTable& 
         if (p <= n) q[p + 1] = make_double2(carry + (s - v) - v * (double)p, v);
         carry += __shfl_sync(0xffffffffu, s, 31);
     }
-    bad = __any_sync(0xffffffffu, bad);
-    if (lane == 0) t.flags[l] = bad;
+    spread.warp();
+    if (lane == 0) t.flags[l] = spread.too_wide((float)n);
 }
 
 // Blocks [0, nset): view tables; the rest: eight lines each of an image's table.
@@ -735,8 +761,10 @@ pix2d_kernel(const Geom2F f, const ViewTables vt, const TI* __restrict__ sino, v
 //     QA_k = sum_{j < k} y_j (bA_{j+1} - bA_j) - y_k bA_k,   QB_k likewise.
 // A pixel's backprojection from the view is S(upper edge) - S(lower edge): one
 // table entry and two FP64 FMAs per edge, whatever the number of columns, with
-// no loop and no divergence.  Sums and differences are FP64, so the table
-// loses nothing against adding the overlaps one by one.  The column of an edge
+// no loop and no divergence.  S is FP64, of up to |y|max times the boundaries'
+// positions in magnitude; rows whose smallest value a difference would lose 2^-18
+// of (Spread::too_wide), and those holding an infinity or a NaN, are walked
+// column by column instead (pix2d_view).  The column of an edge
 // comes from an FP32 position; within that position's error bound of a boundary
 // (RowEps::e, about 1e-4 to 1e-3 columns) the FP64 boundary decides.
 //
@@ -747,9 +775,8 @@ pix2d_kernel(const Geom2F f, const ViewTables vt, const TI* __restrict__ sino, v
 // factor.  A pixel with an edge so close to a boundary that its column is uncertain,
 // or that the boundary may cross the edge by its offset, is walked (pixel_walk).
 //
-// A row holding an infinity or a NaN would spread it over every later entry;
-// such rows are walked column by column instead (pix2d_view), and so are views
-// whose column positions FP32 leaves uncertain by a quarter of a column.
+// Views whose column positions FP32 leaves uncertain by a quarter of a column
+// are walked as well.
 //
 // Entries -1 .. Nu of a row are at [0 .. Nu + 1], in three arrays (a lane's
 // neighbours then load neighbouring words): {QA, QB}, y, and on the arc
@@ -788,8 +815,8 @@ __device__ __forceinline__ RowEps row_eps(const Geom2F& f, const ViewHdr& h, boo
 
 // The table of one detector row (the outer entries continue S as a
 // constant), by a whole CTA of 256 threads; val(j)
-// is the value of traversal column j.  Returns (to all threads) whether the
-// row holds a non-finite value.
+// is the value of traversal column j.  Returns (to all threads) whether the row
+// is to be walked.
 template <typename Val>
 __device__ __forceinline__ bool build_row_table(const ViewTables& vt, const int v, const int Nu, const RowTable e,
                                                 double2* sums, Val&& val) {
@@ -799,7 +826,8 @@ __device__ __forceinline__ bool build_row_table(const ViewTables& vt, const int 
     const float4* ea = vt.arc ? vt.arc + 2 * (size_t)v * (Nu + 1) : nullptr;
     const double nl = (double)(vt.hdr[v].nlines - 1);
     double ca = 0.0, cb = 0.0;  // sums over the columns before this round
-    bool bad = false;
+    Spread spread;
+    float reach = (float)(nl + 1.0);  // positions of pixels and boundaries, on the first and the last line
     if (tid == 0) {
         e.q[0] = make_double2(0.0, 0.0);
         e.y[0] = 0.0f;
@@ -808,10 +836,14 @@ __device__ __forceinline__ bool build_row_table(const ViewTables& vt, const int 
         const int j = base + tid;  // j == Nu: the entry past the end
         float y = 0.0f;
         double a = 0.0, b = 0.0, A = 0.0, B = 0.0;
-        if (j < Nu) {
-            y = val(j);
+        if (j <= Nu) {
             A = bA[j];
             B = bB[j];
+            reach = fmaxf(reach, fmaxf(fabsf((float)A), fabsf((float)fma(B, nl, A))));
+        }
+        if (j < Nu) {
+            y = val(j);
+            spread.add(y);
             if (isfinite(y)) {
                 // (a column whose boundaries are not in order on the lines, a
                 // ray past 90 degrees from the axis, overlaps nothing)
@@ -820,8 +852,6 @@ __device__ __forceinline__ bool build_row_table(const ViewTables& vt, const int 
                     a = (double)y * dA;
                     b = (double)y * dB;
                 }
-            } else {
-                bad = true;
             }
         }
         const double a0 = a, b0 = b;
@@ -849,7 +879,20 @@ __device__ __forceinline__ bool build_row_table(const ViewTables& vt, const int 
             }
         }
     }
-    return __syncthreads_or(bad) != 0;
+    spread.warp();
+    const unsigned far = __reduce_max_sync(0xffffffffu, (unsigned)__float_as_int(reach));
+    uint4* part = reinterpret_cast<uint4*>(sums);
+    __syncthreads();  // the last round's sums are read
+    if (lane == 0) part[wp] = make_uint4(spread.most, spread.least, far, 0u);
+    __syncthreads();
+    unsigned r = 0u;
+    for (int w = 0; w < 8; ++w) {
+        const uint4 p = part[w];
+        spread.most = max(spread.most, p.x);
+        spread.least = min(spread.least, p.y);
+        r = max(r, p.z);
+    }
+    return r >= 0x7f800000u || spread.too_wide(__int_as_float((int)r));
 }
 
 // View tables and row tables of one view per CTA, for all images of the batch.
