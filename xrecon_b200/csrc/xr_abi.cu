@@ -416,7 +416,7 @@ Layout layout(int dim3d, int op, const Geom& g, int nbatch, int nview, int dtype
         const size_t bytes = V * nbatch * (g.Nu + 2) * ROW_ENTRY_BYTES;
         if (bytes <= IL_GROUP_MAX) {
             l.tab = o;    o = align256(o + bytes + 512);  // three arrays, 256-byte aligned each
-            l.flags = o;  o = align256(o + V * nbatch * sizeof(RowEps));
+            l.flags = o;  o = align256(o + V * nbatch * sizeof(float));
         }
     } else if (!dim3d && nbatch == 1 && (op == OP_A || (op == OP_BT && g.type != GEO_ARC))) {
         // line tables (B^T on the arc detector chains its angles, Bw^T weighs
@@ -1065,7 +1065,7 @@ int run2d(int op, const Geom& g, const TI* in, void* out, int dto, const float* 
         const float cw = column_width(g, 0);
         const Geom2F f = make_geom2f(g);
         const RowTable tab = row_table_at(ws + l.tab, (size_t)nview * nbatch * (g.Nu + 2));
-        RowEps* eps = reinterpret_cast<RowEps*>(ws + l.flags);
+        float* eps = reinterpret_cast<float*>(ws + l.flags);
         if (op == OP_AT) table2d_kernel<TI, true><<<nview, 256, 0, st>>>(g, f, ang, nview, vt, in, nbatch, tab, eps);
         else table2d_kernel<TI, false><<<nview, 256, 0, st>>>(g, f, ang, nview, vt, in, nbatch, tab, eps);
         if (int rc = check_cuda("table2d")) return rc;
@@ -1090,7 +1090,7 @@ int run2d(int op, const Geom& g, const TI* in, void* out, int dto, const float* 
         auto kern = op == OP_AT ? pix2t_kernel<TI, OP_AT, false>
                     : vt.arc ? (op == OP_B ? pix2t_kernel<TI, OP_B, true> : pix2t_kernel<TI, OP_BW, true>)
                              : (op == OP_B ? pix2t_kernel<TI, OP_B, false> : pix2t_kernel<TI, OP_BW, false>);
-        if (cudaLaunchKernelEx(&cfg, kern, f, vt, tab, (const RowEps*)eps, in, out, dto, nview, cw, oscale, VS) != cudaSuccess)
+        if (cudaLaunchKernelEx(&cfg, kern, f, vt, tab, (const float*)eps, in, out, dto, nview, cw, oscale, VS) != cudaSuccess)
             return check_cuda("pix2t (cluster launch)");
         return check_cuda("pix2t");
     }
@@ -1792,7 +1792,7 @@ int xr_ragged2d_plan_create(const xr_ragged2d_instance* inst, int ninst, xr_ragg
         L.lflags.push_back(o); o = align256(o + (size_t)(g.W + g.H) * sizeof(int));
         L.filt.push_back(o); o = align256(o + Vs * g.Nu * sizeof(float));
         L.tab.push_back(o);  o = align256(o + Vs * (g.Nu + 2) * ROW_ENTRY_BYTES + 512);
-        L.flags.push_back(o); o = align256(o + Vs * sizeof(RowEps));
+        L.flags.push_back(o); o = align256(o + Vs * sizeof(float));
     }
     for (int l = 0; l < 10; ++l) {
         if (tot[l] > 0x7fffffffll) { delete P; return fail(XR_ERR_UNSUPPORTED, "ragged batch too large"); }
@@ -1851,7 +1851,7 @@ int xr_ragged2d_plan_bind(xr_ragged2d_plan* P, const float* images, float* sino,
         r.sino = sino + in.sino_offset;
         r.filt_out = reinterpret_cast<float*>(ws + L.filt[i]);
         r.tab = row_table_at(ws + L.tab[i], (size_t)in.nview * (r.g.Nu + 2));
-        r.eps = reinterpret_cast<RowEps*>(ws + L.flags[i]);
+        r.eps = reinterpret_cast<float*>(ws + L.flags[i]);
         r.recon = recon + in.img_offset;
         r.ang = angles + in.ang_offset;
         r.filt = filt + in.filt_offset;

@@ -48,7 +48,8 @@ struct Geom2F {
     float dx, dy, inv_dx, inv_dy;
     float sod, shu, du, inv_du, half_nu;
     // error bound of pix2t_view's FP32 column position, in columns: eps0 + eps1
-    // / distance from the source (flat: along the central ray), at most epsw
+    // / distance from the source (flat: along the central ray) of any point of the
+    // 2 x 2 block, at most epsw
     float eps0, eps1, epsw;
     int W, H, Nu, type;
 };
@@ -84,6 +85,9 @@ __host__ __device__ inline Geom2F make_geom2f(const Geom& g) {
     } else {
         e0 += u * 4.3 * r / g.du;
     }
+    // (half as much again: the block is three pixels across, a third of `near`)
+    e1 *= 1.5;
+    if (near < 9.0 * std::max(g.dx, g.dy)) e0 += e1 / near, e1 = 0.0;
     f.eps0 = (float)e0;
     f.eps1 = (float)e1;
     f.epsw = (float)(e0 + e1 / near);
@@ -221,7 +225,9 @@ __device__ __forceinline__ void cell2d_walk(const Geom& g, const Geom2F& f, cons
     const double lim = 1073741824.0, nl = (double)(nlines - 1);
     auto in_lim = [&](double x) { return x > -lim && x < lim; };
     const float dA = (float)(bA1 - bA0), dB = (float)(bB1 - bB0);
-    const bool exact = chain || !(in_lim(bA0) && in_lim(fma(bB0, nl, bA0)) && in_lim(bA1) && in_lim(fma(bB1, nl, bA1))) ||
+    const double q0 = h.q0, q1 = h.q1;
+    const bool behind = !(q0 > 0.0 && fma(q1, nl, q0) > 0.0);  // some lines lie behind the source's plane
+    const bool exact = chain || behind || !(in_lim(bA0) && in_lim(fma(bB0, nl, bA0)) && in_lim(bA1) && in_lim(fma(bB1, nl, bA1))) ||
                        !(fmaxf(fabsf(dA), fabsf(fmaf(dB, (float)nl, dA))) < XR_WIDE2D);
     for (int L = l0; L < nlines; L += ls) {
         const double dL = (double)L;
@@ -243,14 +249,15 @@ __device__ __forceinline__ void cell2d_walk(const Geom& g, const Geom2F& f, cons
             if (pa > pb || !(u1 > 0.0f)) continue;
         } else {
             const double pk1 = fma(bB1, dL, bA1);
+            if (behind && !(fma(q1, dL, q0) > 0.0)) continue;
             pa = max((int)floor(pk), 0);
-            pb = min((int)ceil(pk1) - 1, pb);
+            pb = min(max((int)ceil(pk1), 0) - 1, pb);
             if (pa > pb) continue;
             u0 = (float)(pk - (double)pa);
             u1 = (float)(pk1 - (double)pa);
             u1b = u1;  // upper boundary for the band's later pixels
             if (chain) {
-                const float qd = (float)(fma(h.q1, dL, h.q0) / h.dpix);
+                const float qd = (float)(fma(q1, dL, q0) / h.dpix);
                 u1b = fmaf(d1, qd, u1);
                 u1 = u1b;
                 if (k > 0 && pk > (double)pa)
@@ -258,7 +265,7 @@ __device__ __forceinline__ void cell2d_walk(const Geom& g, const Geom2F& f, cons
             }
         }
         float lf;
-        if (MODE == OP_A) lf = __fdividef(dpixf, (float)fma(h.q1, dL, h.q0));
+        if (MODE == OP_A) lf = __fdividef(dpixf, (float)fma(q1, dL, q0));
         else lf = cw;
         for (int pp = pa; pp <= pb; ++pp) {
             const float o = (float)(pp - pa);
@@ -421,6 +428,20 @@ linetab2d_kernel(const Geom g, const float* __restrict__ ang, const int nview, c
     build_line_table(in + (size_t)b * g.W * g.H, tab, l, threadIdx.x & 31);
 }
 
+// One cell's sum over line L, pixel by pixel: columns from pk to pk1, weight lf per
+// pixel.
+template <typename T>
+__device__ __noinline__ float line_walk(const LineTable& tab, const T* img, bool rows, int L, int npix, double pk, double pk1,
+                                        float lf) {
+    const int pa = max((int)floor(pk), 0), pb = min(max((int)ceil(pk1), 0), npix) - 1;
+    float s = 0.0f;
+    for (int p = pa; p <= pb; ++p) {
+        const float w = (float)(fmin((double)(p + 1), pk1) - fmax((double)p, pk)) * lf;
+        s = fmaf(w, ld(rows ? img + (size_t)L * tab.W + p : img + (size_t)(tab.H - 1 - p) * tab.W + L), s);
+    }
+    return s;
+}
+
 // Cells k and k + 1 (k + 1 < Nu or dropped by the caller) of view v over lines
 // l0, l0 + ls, ...; img is the image itself (flagged lines).
 template <int MODE, typename T>
@@ -440,20 +461,23 @@ __device__ __forceinline__ void cell2t_walk(const Geom2F& f, const ViewTables& v
     const double q0 = h.q0, q1 = h.q1;
     const float dpixf = (float)h.dpix;
     const int* flags = tab.flags + (rows ? 0 : tab.H);
+    // columns whose boundaries are not in order on every line are walked: a
+    // ray past 90 degrees from the axis, or an image with lines behind the
+    // source's plane, which a column overlaps nowhere
+    const double nl = (double)(nlines - 1);
+    bool ordered = true;
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+        ordered = ordered && (k + c >= Nu || (A[c + 1] > A[c] && fma(B[c + 1], nl, A[c + 1]) > fma(B[c], nl, A[c])));
     for (int L = l0; L < nlines; L += ls) {
         const double dL = (double)L;
         float lf = cw;
         if (MODE == OP_A) lf = dpixf * rcp_fast((float)fma(q1, dL, q0));
-        if (flags[L]) {
-#pragma unroll
-            for (int c = 0; c < 2; ++c) {
-                const double pk = fma(B[c], dL, A[c]), pk1 = fma(B[c + 1], dL, A[c + 1]);
-                const int pa = max((int)floor(pk), 0), pb = min((int)ceil(pk1) - 1, npix - 1);
-                for (int p = pa; p <= pb; ++p) {
-                    const float w = (float)(fmin((double)(p + 1), pk1) - fmax((double)p, pk)) * lf;
-                    acc[c] = fmaf(w, ld(rows ? img + (size_t)L * tab.W + p : img + (size_t)(tab.H - 1 - p) * tab.W + L), acc[c]);
-                }
-            }
+        if (flags[L] || !ordered) {
+            if (!(fma(q1, dL, q0) > 0.0)) continue;
+            const double p0 = fma(B[0], dL, A[0]), p1 = fma(B[1], dL, A[1]), p2 = fma(B[2], dL, A[2]);
+            acc[0] += line_walk(tab, img, rows, L, npix, p0, p1, lf);
+            acc[1] += line_walk(tab, img, rows, L, npix, p1, p2, lf);
             continue;
         }
         const double2* q = tab.q + tab.start(rows, L);
@@ -468,18 +492,12 @@ __device__ __forceinline__ void cell2t_walk(const Geom2F& f, const ViewTables& v
         acc[0] = fmaf(lf, (float)(S[1] - S[0]), acc[0]);
         acc[1] = fmaf(lf, (float)(S[2] - S[1]), acc[1]);
     }
-    // a column whose boundaries are not in order on the lines (a ray past 90
-    // degrees from the axis) overlaps nothing
-    const double nl = (double)(nlines - 1);
-#pragma unroll
-    for (int c = 0; c < 2; ++c)
-        if (!(A[c + 1] > A[c]) || !(fma(B[c + 1], nl, A[c + 1]) > fma(B[c], nl, A[c]))) acc[c] = 0.0f;
 }
 
 // A CTA's 8 warps are 8 / LS blocks of 64 columns times LS line slices;
 // blockIdx.z is the image.
 template <typename TI, int MODE>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 4)
 cell2t_kernel(const Geom2F f, const ViewTables vt, LineTable tab, const TI* __restrict__ img, void* __restrict__ sino,
               const int dto, const int nview, const float cw, const int LS) {
     __shared__ float red[8][2][32];
@@ -577,6 +595,7 @@ __device__ __forceinline__ void pix2d_axis(const Geom2F& f, const ViewTables& vt
         const float ya = USE_X ? fmaf(-Lf, f.dy, f.yc0) : fmaf((float)p0, f.dy, f.y0);
         float lf = cw, q = 1.0f;
         if (MODE == OP_AT || chain) q = (float)fma(q1, dL, q0);
+        if (!(fma(q1, dL, q0) > 0.0)) continue;  // behind the source's plane
         if (MODE == OP_AT) lf = __fdividef(USE_X ? f.dx : f.dy, q);
         const float kf = guess(xa, ya) - XR_GUESS2D;
         if (kf >= (float)Nu) continue;
@@ -644,7 +663,7 @@ __device__ __forceinline__ void pix2d_axis(const Geom2F& f, const ViewTables& vt
         auto upper = [&](float lower) -> float {  // boundary k + 1 from boundary k
             W = wr[k];
             const float w = fmaf(W.y, Lf, W.x);
-            return w < XR_WIDE2D ? lower + w : (float)(fma(bB[k + 1], dL, bA[k + 1]) - dp);
+            return fabsf(w) < XR_WIDE2D ? lower + w : (float)(fma(bB[k + 1], dL, bA[k + 1]) - dp);
         };
         auto value = [&]() -> Lanes<NB> {
             Lanes<NB> y = src(col_of(k));
@@ -766,7 +785,7 @@ pix2d_kernel(const Geom2F f, const ViewTables vt, const TI* __restrict__ sino, v
 // of (Spread::too_wide), and those holding an infinity or a NaN, are walked
 // column by column instead (pix2d_view).  The column of an edge
 // comes from an FP32 position; within that position's error bound of a boundary
-// (RowEps::e, about 1e-4 to 1e-3 columns) the FP64 boundary decides.
+// (row_eps, about 1e-4 to 1e-3 columns) the FP64 boundary decides.
 //
 // On the arc detector B and Bw walk each pixel's columns with float32 angles
 // chained from its first column (ArcChain): boundary j inside the pixel lies
@@ -794,32 +813,29 @@ constexpr size_t ROW_ENTRY_BYTES = sizeof(double2) + sizeof(float) + sizeof(floa
 constexpr int PT_MAX_BATCH = 4;
 
 // Of a row: error bound of its view's column positions without the distance
-// term (columns; ROW_WALK: the row is walked), and the rounding of a boundary
-// angle (columns; arc detector).
-struct RowEps {
-    float e, q;
-};
+// term (columns; ROW_WALK: the row is walked).  `steps` bounds the columns of a
+// pixel where chained angles are walked (0: none): a boundary is then up to steps +
+// 3 roundings off its direct angle.
 constexpr float ROW_WALK = 2.0f;
-
-__device__ __forceinline__ RowEps row_eps(const Geom2F& f, const ViewHdr& h, bool bad) {
-    RowEps r{f.eps0, 0.0f};
+__device__ __forceinline__ float row_eps(const Geom2F& f, const ViewHdr& h, float steps) {
+    float q = 0.0f;
     if (f.type == GEO_ARC) {
         // half a unit of the largest angle: 2^-24 of its power of two
         const float a = fabsf((float)h.beta) + fabsf(f.shu) + f.half_nu * f.du;
-        r.q = __int_as_float((__float_as_int(fmaxf(a, 1.0e-6f)) & 0x7f800000) - (24 << 23)) * f.inv_du;
-        r.e += 1.1f * r.q;
+        q = __int_as_float((__float_as_int(fmaxf(a, 1.0e-6f)) & 0x7f800000) - (24 << 23)) * f.inv_du;
+        q *= 1.1f + (steps > 0.0f ? steps + 3.0f : 0.0f);
     }
-    if (bad || !(f.epsw + 1.1f * r.q < 0.25f)) r.e = ROW_WALK;
-    return r;
+    return f.epsw + q < 0.25f ? f.eps0 + q : ROW_WALK;
 }
 
 // The table of one detector row (the outer entries continue S as a
 // constant), by a whole CTA of 256 threads; val(j)
-// is the value of traversal column j.  Returns (to all threads) whether the row
-// is to be walked.
+// is the value of traversal column j.  Returns (to all threads) the row's error
+// bound (row_eps).
 template <typename Val>
-__device__ __forceinline__ bool build_row_table(const ViewTables& vt, const int v, const int Nu, const RowTable e,
-                                                double2* sums, Val&& val) {
+__device__ __forceinline__ float build_row_table(const Geom2F& f, const ViewTables& vt, const int v, const RowTable e,
+                                                 double2* sums, Val&& val) {
+    const int Nu = f.Nu;
     const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
     const double* bA = vt.bA + (size_t)v * (Nu + 1);
     const double* bB = vt.bB + (size_t)v * (Nu + 1);
@@ -828,6 +844,7 @@ __device__ __forceinline__ bool build_row_table(const ViewTables& vt, const int 
     double ca = 0.0, cb = 0.0;  // sums over the columns before this round
     Spread spread;
     float reach = (float)(nl + 1.0);  // positions of pixels and boundaries, on the first and the last line
+    float width = 3.0e38f;            // narrowest column there
     if (tid == 0) {
         e.q[0] = make_double2(0.0, 0.0);
         e.y[0] = 0.0f;
@@ -844,15 +861,12 @@ __device__ __forceinline__ bool build_row_table(const ViewTables& vt, const int 
         if (j < Nu) {
             y = val(j);
             spread.add(y);
+            const double dA = bA[j + 1] - A, dB = bB[j + 1] - B;
             if (isfinite(y)) {
-                // (a column whose boundaries are not in order on the lines, a
-                // ray past 90 degrees from the axis, overlaps nothing)
-                const double dA = bA[j + 1] - A, dB = bB[j + 1] - B;
-                if (dA > 0.0 && fma(dB, nl, dA) > 0.0) {
-                    a = (double)y * dA;
-                    b = (double)y * dB;
-                }
+                a = (double)y * dA;
+                b = (double)y * dB;
             }
+            width = fminf(width, fminf((float)dA, (float)fma(dB, nl, dA)));
         }
         const double a0 = a, b0 = b;
 #pragma unroll
@@ -880,26 +894,32 @@ __device__ __forceinline__ bool build_row_table(const ViewTables& vt, const int 
         }
     }
     spread.warp();
+    // boundaries out of order on a line (a ray past 90 degrees from the axis; lines
+    // behind the source's plane): S would run back there
+    if (!(width > 0.0f)) reach = __int_as_float(0x7f800000);
     const unsigned far = __reduce_max_sync(0xffffffffu, (unsigned)__float_as_int(reach));
+    const unsigned thin = __reduce_min_sync(0xffffffffu, (unsigned)__float_as_int(fmaxf(width, 0.0f)));
     uint4* part = reinterpret_cast<uint4*>(sums);
     __syncthreads();  // the last round's sums are read
-    if (lane == 0) part[wp] = make_uint4(spread.most, spread.least, far, 0u);
+    if (lane == 0) part[wp] = make_uint4(spread.most, spread.least, far, thin);
     __syncthreads();
-    unsigned r = 0u;
+    unsigned r = 0u, t = 0xffffffffu;
     for (int w = 0; w < 8; ++w) {
         const uint4 p = part[w];
         spread.most = max(spread.most, p.x);
         spread.least = min(spread.least, p.y);
         r = max(r, p.z);
+        t = min(t, p.w);
     }
-    return r >= 0x7f800000u || spread.too_wide(__int_as_float((int)r));
+    if (r >= 0x7f800000u || spread.too_wide(__int_as_float((int)r))) return ROW_WALK;
+    return row_eps(f, vt.hdr[v], vt.arc ? 2.0f + 1.0f / __int_as_float((int)t) : 0.0f);
 }
 
 // View tables and row tables of one view per CTA, for all images of the batch.
 template <typename TI, bool SCALE>
 __global__ void __launch_bounds__(256)
 table2d_kernel(const Geom g, const Geom2F f, const float* __restrict__ ang, const int nview, const ViewTables vt,
-               const TI* __restrict__ sino, const int nbatch, const RowTable tab, RowEps* __restrict__ eps) {
+               const TI* __restrict__ sino, const int nbatch, const RowTable tab, float* __restrict__ eps) {
     __shared__ double2 sums[8];
     const int v = blockIdx.x, Nu = g.Nu;
     for (int k = threadIdx.x; k <= Nu; k += 256) setup_view_entry(g, 0, ang[v], v, k, vt, g.type == GEO_ARC);
@@ -908,11 +928,11 @@ table2d_kernel(const Geom g, const Geom2F f, const float* __restrict__ ang, cons
     for (int b = 0; b < nbatch; ++b) {
         const size_t row = (size_t)b * nview + v;
         const TI* y = sino + row * Nu;
-        const bool bad = build_row_table(vt, v, Nu, tab.at(row, Nu), sums, [&](int j) -> float {
+        const float e = build_row_table(f, vt, v, tab.at(row, Nu), sums, [&](int j) -> float {
             const float x = ld(y + (keep ? j : Nu - 1 - j));
             return SCALE ? x * vt.colE[(size_t)v * Nu + j] : x;
         });
-        if (threadIdx.x == 0) eps[row] = row_eps(f, vt.hdr[v], bad);
+        if (threadIdx.x == 0) eps[row] = e;
     }
 }
 
@@ -965,7 +985,7 @@ __device__ __noinline__ float pixel_walk(const Geom2F& f, const ViewTables& vt, 
 // may cross an edge.
 template <int MODE, bool CHAIN>
 __device__ __forceinline__ unsigned pix2t_view(const Geom2F& f, const ViewTables& vt, const int v, const int ix0,
-                                           const int iy0, const float cw, const RowTable tab, const RowEps eps,
+                                           const int iy0, const float cw, const RowTable tab, const float eps,
                                            float (&acc)[P2][P2]) {
     const ViewHdr* h = vt.hdr + v;
     const int4 hi = *reinterpret_cast<const int4*>(&h->use_x);
@@ -978,9 +998,9 @@ __device__ __forceinline__ unsigned pix2t_view(const Geom2F& f, const ViewTables
     const float y0 = use_x ? fmaf(-(float)L0, f.dy, f.yc0) : fmaf((float)p0, f.dy, f.y0);
     const float ex = use_x ? f.dx : 0.0f, ey = use_x ? 0.0f : f.dy;
     const float lx = use_x ? 0.0f : f.dx, ly = use_x ? -f.dy : 0.0f;
-    // column coordinate = u sg + k0f
+    // column coordinate, less a half = u sg + k0f
     const float sg = keep ? f.inv_du : -f.inv_du;
-    const float k0f = f.half_nu - (f.type == GEO_ARC ? 0.0f : f.shu * sg);
+    const float k0f = f.half_nu - 0.5f - (f.type == GEO_ARC ? 0.0f : f.shu * sg);
     float t[P2][P2];
     unsigned walk = 0;  // pixels to walk, bit j P2 + i
 #pragma unroll
@@ -989,7 +1009,7 @@ __device__ __forceinline__ unsigned pix2t_view(const Geom2F& f, const ViewTables
         const float xa = fmaf((float)j, lx, x0), ya = fmaf((float)j, ly, y0);
         double S[P2 + 1];
         int ki[P2 + 1];  // entry of each edge's column (0: before the first)
-        float off[P2 + 1], em = 0.0f;  // distance of each edge from its column's middle, the edges' error bound
+        float off[P2 + 1], lim = 0.5f;  // offset of each edge from its column's middle; above lim its column is uncertain
 #pragma unroll
         for (int i = 0; i <= P2; ++i) {
             const float x = fmaf((float)i, ex, xa), y = fmaf((float)i, ey, ya);
@@ -1003,21 +1023,21 @@ __device__ __forceinline__ unsigned pix2t_view(const Geom2F& f, const ViewTables
             } else {
                 u = x * hs.y + y * hs.x;
             }
-            // (half a column outside the detector is as good as any place there)
-            const float kf = fminf(fmaxf(fmaf(u, sg, k0f), -0.5f), (float)Nu + 0.5f);
-            // floor by an add of 1.5 * 2^23 rounded down: the column in the low bits
-            const float tr = __fadd_rd(kf, 12582912.0f);
+            if (i == 0) lim -= fmaf(f.eps1, inv, eps);
+            // (a place outside the detector is as good as any there)
+            const float kf = fminf(fmaxf(fmaf(u, sg, k0f), -1.0f), (float)Nu);
+            // rounded by an add of 1.5 * 2^23: the column in the low bits
+            const float tr = kf + 12582912.0f;
             ki[i] = XR_BOUND((__float_as_int(tr) - 0x4B400000) + 1, 0, Nu + 1);
-            off[i] = (kf - (tr - 12582912.0f)) - 0.5f;
-            em = fmaxf(em, fmaf(f.eps1, inv, eps.e));
+            off[i] = kf - (tr - 12582912.0f);
         }
-        bool near = false;
+        bool near[P2 + 1];
 #pragma unroll
-        for (int i = 0; i <= P2; ++i) near = near || fabsf(off[i]) > 0.5f - em;
-        if (!CHAIN && near) {
+        for (int i = 0; i <= P2; ++i) near[i] = fabsf(off[i]) > lim;
+        if (!CHAIN && (near[0] || near[1] || near[2])) {
 #pragma unroll
             for (int i = 0; i <= P2; ++i)
-                if (fabsf(off[i]) > 0.5f - em) {  // boundary b decides
+                if (near[i]) {  // boundary b decides
                     const int b = XR_BOUND(ki[i] - 1 + (off[i] > 0.0f), 0, Nu);
                     const size_t ob = (size_t)v * (Nu + 1) + b;
                     ki[i] = b + (fma(vt.bB[ob], dL, vt.bA[ob]) <= (double)(p0 + i));
@@ -1039,11 +1059,9 @@ __device__ __forceinline__ unsigned pix2t_view(const Geom2F& f, const ViewTables
             if (MODE == OP_AT) s *= lf;
             if (CHAIN) {
                 // boundaries ka + 1 .. kb (entries ka + 2 ..) lie in the pixel;
-                // the walk starts at column ka.  A boundary's offset is up to
-                // steps + 3 roundings.
-                const float ec = fmaf((float)(ki[i + 1] - ki[i] + 3), eps.q, em);
+                // the walk starts at column ka
                 const int ka = max(ki[i] - 1, 0), kb = min(ki[i + 1] - 1, Nu);
-                if (off[i] < em - 0.5f || off[i] > 0.5f - ec || fabsf(off[i + 1]) > 0.5f - ec) {
+                if (near[i] || near[i + 1]) {
                     s = 0.0f;
                     walk |= 1u << (use_x ? j * P2 + i : (P2 - 1 - i) * P2 + j);
                 } else if (kb > ka) {
@@ -1089,7 +1107,7 @@ __device__ __forceinline__ unsigned pix2t_view(const Geom2F& f, const ViewTables
 // once, a warp would wait for one of them in most views of an arc scan: a ragged
 // batch of 16 arc scans 14488 -> 12028 us).
 template <int MODE, bool CHAIN, typename Src>
-__device__ __forceinline__ void pix2t_views(const Geom2F& f, const ViewTables& vt, const RowTable tab, const RowEps* eps,
+__device__ __forceinline__ void pix2t_views(const Geom2F& f, const ViewTables& vt, const RowTable tab, const float* eps,
                                             const int ix0, const int iy0, const float cw, const int v0, const int nview,
                                             const int vs, Src&& src, float (&acc)[P2][P2]) {
     constexpr int CAP = 16;
@@ -1106,8 +1124,8 @@ __device__ __forceinline__ void pix2t_views(const Geom2F& f, const ViewTables& v
         n = 0;
     };
     for (int v = v0; v < nview; v += vs) {
-        const RowEps e = eps[v];
-        if (e.e >= 1.0f) {
+        const float e = eps[v];
+        if (e >= 1.0f) {
             const float4 s = pix2d_view_walk<MODE>(f, vt, v, ix0, iy0, cw, src(v));
             acc[0][0] += s.x; acc[0][1] += s.y; acc[1][0] += s.z; acc[1][1] += s.w;
             continue;
@@ -1144,7 +1162,7 @@ __device__ __forceinline__ void pix2t_origin(const Geom2F& f, int VS, int cta, i
 template <typename TI, int MODE, bool CHAIN>
 __global__ void __launch_bounds__(256, 4)
 pix2t_kernel(const __grid_constant__ Geom2F f, const __grid_constant__ ViewTables vt, const RowTable tab,
-             const RowEps* __restrict__ eps, const TI* __restrict__ sino, void* __restrict__ img, const int dto,
+             const float* __restrict__ eps, const TI* __restrict__ sino, void* __restrict__ img, const int dto,
              const int nview, const float cw, const float oscale, const int VS) {
     namespace cg = cooperative_groups;
     __shared__ float red[8][P2 * P2][32];

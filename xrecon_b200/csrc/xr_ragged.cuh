@@ -45,7 +45,7 @@ struct RaggedDev {
     float* sino;
     float* filt_out;
     RowTable tab;   // row tables of filt_out and their error bounds (xr_dd2d.cuh)
-    RowEps* eps;
+    float* eps;
     float* recon;
     const float* ang;
     const float* filt;
@@ -197,9 +197,9 @@ ragged2d_fbp_kernel(const RaggedDev* __restrict__ inst, const int ninst, const i
         __syncthreads();  // the whole row is in filt_out
         const float* y = I.filt_out + (size_t)v * Nu;
         const int keep = I.vt.hdr[v].keep;
-        const bool bad = build_row_table(I.vt, v, Nu, I.tab.at(v, Nu), row_sums,
-                                         [&](int j) -> float { return y[keep ? j : Nu - 1 - j]; });
-        if (tid == 0) I.eps[v] = row_eps(I.f, I.vt.hdr[v], bad);
+        const float e = build_row_table(I.f, I.vt, v, I.tab.at(v, Nu), row_sums,
+                                        [&](int j) -> float { return y[keep ? j : Nu - 1 - j]; });
+        if (tid == 0) I.eps[v] = e;
     }
     if (!grid_barrier(bar, nb)) return;
 
