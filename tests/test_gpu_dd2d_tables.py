@@ -174,3 +174,23 @@ def test_lines_behind_the_source_plane_in_a_ragged_batch(cuda):
     sino, recon = RaggedFBP2d([P], [ang])([img.to(cuda)])
     assert rel_l2(sino[0].cpu().numpy(), O.dd2d("A", img.numpy(), P.options.cpu().numpy(), ang.numpy())) < 1e-5
     assert rel_l2(recon[0].cpu().numpy(), P.filtered_backprojection(sino[0], ang.to(cuda)).cpu().numpy()) < 1e-5
+
+
+@pytest.mark.parametrize("du,n,x", [(2e-7, 600, 0.0), (5e-8, 600, 0.0), (3e-7, 2200000, 150.0)])
+@pytest.mark.parametrize("B", [1, 8])
+def test_columns_finer_than_the_guess(cuda, du, n, x, B):
+    """Arc columns of less than the column guess's error in radians (2e-6 towards x = 150 mm), at view angles that
+    float32 resolves: every column is found, whichever way the batch is gathered (1e-5, the bound of every
+    operator).  Towards x = 150 mm only A^T: the angles' float32 unit there is a tenth of a column, and the chained
+    operators' own roundings are 1.6e-4 whatever finds the column."""
+    sod = 500.0
+    opts = _opts("arc", 24, 20, n, du * 1000.0, sod, 1000.0, (x, 0.0, 0.0))
+    opts[3:5] = 0.7 * 600 * du * sod / 24
+    ang = np.array([0.01, -0.008], np.float32)
+    sino = np.random.default_rng(7).random((B, 1, 2, n), dtype=np.float32)
+    sino[0, 0, 1, n // 2] = np.inf if B == 1 else 1.0  # one image: a walked row among tabled ones
+    for op in ("AT", "B", "BW") if x == 0.0 else ("AT",):
+        want = O.dd2d(op, sino, opts, ang)
+        ok = np.isfinite(want)
+        got = _run(op, sino, opts, ang, cuda).cpu().numpy()
+        assert rel_l2(got[ok], want[ok]) < 1e-5, op

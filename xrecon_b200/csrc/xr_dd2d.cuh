@@ -51,6 +51,7 @@ struct Geom2F {
     // / distance from the source (flat: along the central ray) of any point of the
     // 2 x 2 block, at most epsw
     float eps0, eps1, epsw;
+    float guess;  // error bound of pix2d_axis's column guess, in columns
     int W, H, Nu, type;
 };
 
@@ -91,6 +92,7 @@ __host__ __device__ inline Geom2F make_geom2f(const Geom& g) {
     f.eps0 = (float)e0;
     f.eps1 = (float)e1;
     f.epsw = (float)(e0 + e1 / near);
+    f.guess = f.epsw + (g.type == GEO_ARC ? XR_GUESS_ATAN_ERR * f.inv_du : 0.0f);
     f.W = g.W; f.H = g.H; f.Nu = g.Nu; f.type = g.type;
     return f;
 }
@@ -532,7 +534,6 @@ cell2t_kernel(const Geom2F f, const ViewTables vt, LineTable tab, const TI* __re
 // ----------------------------------------------------------- pixel gather
 
 constexpr int P2 = 2;                  // pixels per side of a thread's block
-constexpr float XR_GUESS2D = 0.0625f;  // columns; above the guesses' FP32 error
 
 // NB images' sinogram values of one column of one view.
 template <typename TI, int NB>
@@ -556,7 +557,7 @@ struct SinoLanes {
 // run of P2 pixels in the line's pixel coordinates, relative to the run's
 // start: each overlap is weighted with the line factor and cell scale (A^T) or
 // the column width (B; times the FBP weight for Bw).  The run's first column is
-// guessed in FP32 at its lower edge, a sixteenth of a column low, and corrected
+// guessed in FP32 at its lower edge, low by the guess's error bound, and corrected
 // against the tables, so the guess decides no result.  Its lower boundary is
 // FP64; the next ones add the columns' FP32 widths on the line (columns wider
 // than XR_WIDE2D: FP64 as well).
@@ -584,6 +585,8 @@ __device__ __forceinline__ void pix2d_axis(const Geom2F& f, const ViewTables& vt
         }
         return keep ? f.half_nu + u : f.half_nu - u;
     };
+    // (float32 boundary angles: half a unit of the view's own)
+    const float margin = f.type == GEO_ARC ? fmaf(fabsf((float)h->beta) * 5.9604645e-8f, f.inv_du, f.guess) : f.guess;
     const int p0 = USE_X ? ix0 : f.H - P2 - iy0;  // first pixel of the runs
     const double dp = (double)p0;
 #pragma unroll
@@ -597,14 +600,14 @@ __device__ __forceinline__ void pix2d_axis(const Geom2F& f, const ViewTables& vt
         if (MODE == OP_AT || chain) q = (float)fma(q1, dL, q0);
         if (!(fma(q1, dL, q0) > 0.0)) continue;  // behind the source's plane
         if (MODE == OP_AT) lf = __fdividef(USE_X ? f.dx : f.dy, q);
-        const float kf = guess(xa, ya) - XR_GUESS2D;
+        const float kf = guess(xa, ya) - margin;
         if (kf >= (float)Nu) continue;
         if (kf < 0.0f &&
-            guess(USE_X ? fmaf((float)P2, f.dx, xa) : xa, USE_X ? ya : fmaf((float)P2, f.dy, ya)) + XR_GUESS2D < 0.0f)
+            guess(USE_X ? fmaf((float)P2, f.dx, xa) : xa, USE_X ? ya : fmaf((float)P2, f.dy, ya)) + margin < 0.0f)
             continue;
         int k = (int)fminf(fmaxf(kf, 0.0f), (float)(Nu - 1));
         float pk0 = (float)(fma(bB[k], dL, bA[k]) - dp);
-        for (int i = 0; i < 2 && pk0 > 0.0f && k > 0; ++i) {
+        while (pk0 > 0.0f && k > 0) {
             --k;
             pk0 = (float)(fma(bB[k], dL, bA[k]) - dp);
         }
