@@ -788,6 +788,20 @@ CellPlans plan_cell_helical(const Geom& g) {
     return plan_cell_shapes(gp, g.D + 2);
 }
 
+// The unstaged gather; CS: the split that the staged one would take, followed
+// for float32 outputs.
+template <typename TO, int MODE, bool HEL, bool CHAIN>
+int launch_vox_prefix(const Geom& g, const GeomF& gf, const ViewTables& vt, const float2* tab, TO* out, int nbatch, int nview,
+                      int nzp, cudaStream_t st, double z0dz, double zd0, double dvv, float cw, float atconst, float oscale,
+                      int CS) {
+    const dim3 grid((g.W + 31) / 32, (g.H + PFX_NWY - 1) / PFX_NWY, nzp * nbatch), block(32, PFX_NWY);
+    auto kern = vox_prefix3d_kernel<TO, PFX_R, PFX_NWY, MODE, HEL, CHAIN>;
+    if constexpr (std::is_same<TO, float>::value)
+        if (CS > 1) kern = vox_prefix3d_kernel<TO, PFX_R, PFX_NWY, MODE, HEL, CHAIN, true>;
+    kern<<<grid, block, 0, st>>>(g, gf, vt, tab, out, nview, nzp, z0dz, zd0, dvv, cw, atconst, oscale, CS);
+    return check_cuda("vox_prefix3d");
+}
+
 template <bool HEL = false, typename TO>
 int run_cell_tma(int eff, const Geom& g, const float* in, TO* out, int nbatch, int nview, char* ws,
                  const Layout& l, const ViewTables& vt, cudaStream_t st, double z0dz, double zd0, double dvv, float cw,
@@ -922,25 +936,17 @@ int run3d(int op, const Geom& g, const TI* in, TO* out, const float* ang, int nb
             if (rc >= 0) return rc;
         }
         const PfxStagePlan sp = plan_pfx_stage(g);
-        const int CS = sp.ok ? pfx_split(g, nbatch, nview, nzp, sp.BC, sp.BR) : 1;  // sums in the staged gather's order
-        dim3 pgrid((g.W + 31) / 32, (g.H + PFX_NWY - 1) / PFX_NWY, nzp * nbatch);
-        dim3 pblock(32, PFX_NWY);
-        if (eff == OP_AT)
-            vox_prefix3d_kernel<TO, PFX_R, PFX_NWY, OP_AT><<<pgrid, pblock, 0, st>>>(
-                g, gf, vt, tab, out, nview, nzp, z0dz, zd0, dvv, cw, atconst, oscale, CS);
-        else if (vt.arc && eff == OP_B)
-            vox_prefix3d_kernel<TO, PFX_R, PFX_NWY, OP_B, false, true><<<pgrid, pblock, 0, st>>>(
-                g, gf, vt, tab, out, nview, nzp, z0dz, zd0, dvv, cw, atconst, oscale, CS);
-        else if (vt.arc)
-            vox_prefix3d_kernel<TO, PFX_R, PFX_NWY, OP_BW, false, true><<<pgrid, pblock, 0, st>>>(
-                g, gf, vt, tab, out, nview, nzp, z0dz, zd0, dvv, cw, atconst, oscale, CS);
-        else if (eff == OP_B)
-            vox_prefix3d_kernel<TO, PFX_R, PFX_NWY, OP_B><<<pgrid, pblock, 0, st>>>(
-                g, gf, vt, tab, out, nview, nzp, z0dz, zd0, dvv, cw, atconst, oscale, CS);
-        else
-            vox_prefix3d_kernel<TO, PFX_R, PFX_NWY, OP_BW><<<pgrid, pblock, 0, st>>>(
-                g, gf, vt, tab, out, nview, nzp, z0dz, zd0, dvv, cw, atconst, oscale, CS);
-        return check_cuda("vox_prefix3d");
+        const int CS = sp.ok ? pfx_split(g, nbatch, nview, nzp, sp.BC, sp.BR) : 1;
+        auto launch = [&](auto mode, auto chain) {
+            return launch_vox_prefix<TO, decltype(mode)::value, false, decltype(chain)::value>(
+                g, gf, vt, tab, out, nbatch, nview, nzp, st, z0dz, zd0, dvv, cw, atconst, oscale, CS);
+        };
+        if (eff == OP_AT) return launch(std::integral_constant<int, OP_AT>{}, std::false_type{});
+        if (eff == OP_B)
+            return vt.arc ? launch(std::integral_constant<int, OP_B>{}, std::true_type{})
+                          : launch(std::integral_constant<int, OP_B>{}, std::false_type{});
+        return vt.arc ? launch(std::integral_constant<int, OP_BW>{}, std::true_type{})
+                      : launch(std::integral_constant<int, OP_BW>{}, std::false_type{});
     }
     if (eff == OP_AT) {
         if (g.type != GEO_PARALLEL) {
@@ -1330,8 +1336,6 @@ int helical(int op, const Geom& g, const HelOpts& o, const float* in, float* out
     }
     const int nzp = (g.D + PFX_R - 1) / PFX_R;
     if ((long long)nzp * nbatch > 65535) return fail(XR_ERR_UNSUPPORTED, "depth x batch too large for one launch");
-    dim3 pgrid((g.W + 31) / 32, (g.H + PFX_NWY - 1) / PFX_NWY, nzp * nbatch);
-    dim3 pblock(32, PFX_NWY);
     const float atconst = (float)(g.dx * g.dy * g.dz / (g.du * g.dv));
     // the table footprints staged in shared memory (the box from the plan of
     // the same volume and detector on a circular scan; views whose box does
@@ -1342,14 +1346,11 @@ int helical(int op, const Geom& g, const HelOpts& o, const float* in, float* out
         if (rc >= 0) return rc;
     }
     const PfxStagePlan plan = plan_pfx_stage(g);
-    const int CS = plan.ok ? pfx_split(g, nbatch, nview, nzp, plan.BC, plan.BR) : 1;  // sums in the staged gather's order
-    if (op == OP_AT)
-        vox_prefix3d_kernel<float, PFX_R, PFX_NWY, OP_AT, true><<<pgrid, pblock, 0, st>>>(
-            g, gf, vt, tab, out, nview, nzp, z0dz, zd0, dvv, 0.0f, atconst, 1.0f, CS);
-    else
-        vox_prefix3d_kernel<float, PFX_R, PFX_NWY, OP_B, true><<<pgrid, pblock, 0, st>>>(
-            g, gf, vt, tab, out, nview, nzp, z0dz, zd0, dvv, 0.0f, atconst, 1.0f, CS);
-    return check_cuda("vox_prefix3d");
+    const int CS = plan.ok ? pfx_split(g, nbatch, nview, nzp, plan.BC, plan.BR) : 1;
+    return op == OP_AT ? launch_vox_prefix<float, OP_AT, true, false>(g, gf, vt, tab, out, nbatch, nview, nzp, st, z0dz, zd0,
+                                                                      dvv, 0.0f, atconst, 1.0f, CS)
+                       : launch_vox_prefix<float, OP_B, true, false>(g, gf, vt, tab, out, nbatch, nview, nzp, st, z0dz, zd0,
+                                                                     dvv, 0.0f, atconst, 1.0f, CS);
 }
 
 // ------------------------------------------------------ ragged 2D batches

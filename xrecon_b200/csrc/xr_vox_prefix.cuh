@@ -114,7 +114,12 @@ __device__ __forceinline__ float col_guess_fast(const GeomF& gf, const ViewHdr& 
 //   CHAIN      : circular arc detector, B / Bw: the pixel's columns are
 //                walked with the reference's chained float32 angles
 //                (ArcChain, vt.arc)
-template <typename TO, int R, int NWY, int MODE, bool HEL = false, bool CHAIN = false>
+//   SPLIT      : the views' sums taken as the staged gather takes them when it
+//                splits them over CS CTAs (views r, r + CS, ... first, then over
+//                r), for comparing the two bit for bit; an instance of its own,
+//                since the second set of sums spills (64 to 112 bytes a thread at
+//                64 registers, against 0 to 12)
+template <typename TO, int R, int NWY, int MODE, bool HEL = false, bool CHAIN = false, bool SPLIT = false>
 __global__ void __launch_bounds__(32 * NWY, XR_PFX_MINB)
 vox_prefix3d_kernel(const Geom g, const GeomF gf, const ViewTables vt, const float2* __restrict__ tab,
                     TO* __restrict__ vol, const int nview, const int nzg, const double z0dz, const double zd0,
@@ -141,12 +146,10 @@ vox_prefix3d_kernel(const Geom g, const GeomF gf, const ViewTables vt, const flo
 #pragma unroll
     for (int i = 0; i < R; ++i) acc[i] = 0.0f;
 
-    // CS > 1: the views' sums taken as the staged gather takes them when it
-    // splits them over CS CTAs (views r, r + CS, ... first, then over r)
-    float sums[R];
+    float sums[SPLIT ? R : 1];
 #pragma unroll 1
-    for (int r = 0; r < CS; ++r) {
-    for (int v = r; v < nview; v += CS) {
+    for (int r = 0; r < (SPLIT ? CS : 1); ++r) {
+    for (int v = r; v < nview; v += SPLIT ? CS : 1) {
         const ViewHdr& h = vt.hdr[v];
         const int keep = h.keep;
         float cwv = cw;
@@ -346,12 +349,12 @@ vox_prefix3d_kernel(const Geom g, const GeomF gf, const ViewTables vt, const flo
             }
         }
     }
-    if (CS == 1) break;
+    if constexpr (SPLIT)
 #pragma unroll
-    for (int i = 0; i < R; ++i) {
-        sums[i] = r ? sums[i] + acc[i] : acc[i];
-        acc[i] = r + 1 < CS ? 0.0f : sums[i];
-    }
+        for (int i = 0; i < R; ++i) {
+            sums[i] = r ? sums[i] + acc[i] : acc[i];
+            acc[i] = r + 1 < CS ? 0.0f : sums[i];
+        }
     }
 #pragma unroll
     for (int i = 0; i < R; ++i) {

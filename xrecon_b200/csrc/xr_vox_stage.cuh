@@ -196,7 +196,8 @@ __global__ void __launch_bounds__(PS_T * PS_T, XR_PFXS_MINB)
 vox_stage3d_kernel(const Geom g, const GeomF gf, const ViewTables vt, const __grid_constant__ CUtensorMap map,
                    const float2* __restrict__ tab, TO* __restrict__ vol, int* __restrict__ unfit, const int nview,
                    const int nzg, const double z0dz, const double zd0, const double dvv, const float cw,
-                   const float atconst, const float oscale, const int BC, const int BR, const int CS) {
+                   const float atconst, const float oscale, const int BC, const int BR, const int CS_) {
+    const int CS = FALLBACK ? 1 : CS_;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     int4* wins = reinterpret_cast<int4*>(smem_raw);
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw + 2 * PS_WCH * sizeof(int4));
