@@ -220,24 +220,23 @@ CellPlans plan_cell_shapes(const Geom& g, int cap_z) {
     const double rs = (g.type == GEO_FLAT) ? g.sod / g.sdd : 1.0;
     const double zd0 = (-0.5 * g.Nv * g.dv + g.shv) * rs, dvv = g.dv * rs;
     const double z0dz = (-0.5 * g.D * g.dz + g.shz) / g.dz;
-    // rows per CTA: the default shape's, and that of every shape the launch may take
-    CellPlan def{false, 0, 0, cell_rows_per_thread(g), CELL_NW, false, 2};
-    int shapes[3][2] = {{def.R, def.NW}, {0, 0}, {0, 0}};
-    cell_shape(g.Nv, false, shapes[1][0], shapes[1][1]);
-    cell_shape(g.Nv, true, shapes[2][0], shapes[2][1]);
-    int maxspan = 0;
-    double maxnz[3] = {0.0, 0.0, 0.0};
     std::vector<double> A(g.Nu + 1), B(g.Nu + 1), Q(g.Nu);
     std::vector<double> angles;
+    // the CTAs' column blocks of every sampled view, for the windows below
+    const int nblk = (g.Nu + 31) / 32;
+    std::vector<ViewHdr> views;
+    std::vector<CellCtaGeo> blocks;
     const int NSA = 256;
     for (int i = 0; i < NSA; ++i) angles.push_back(2.0 * M_PI * i / NSA + 0.37 / NSA);
     for (int i = 0; i < 8; ++i) {
         angles.push_back(M_PI / 4 * i + 1e-5);
         angles.push_back(M_PI / 4 * i - 1e-5);
     }
-    for (double ang : angles) {
+    views.reserve(angles.size());
+    blocks.reserve(angles.size() * nblk);
+    for (size_t a = 0; a < angles.size(); ++a) {
         ViewHdr h;
-        make_view_hdr(g, (float)ang, h);
+        make_view_hdr(g, (float)angles[a], h);
         for (int k = 0; k <= g.Nu; ++k) {
             const double D = boundary_axis(g, h, (double)k, uscale);
             boundary_line_coeffs(g, h, D, A[k], B[k]);
@@ -257,33 +256,22 @@ CellPlans plan_cell_shapes(const Geom& g, int cap_z) {
                     return (std::max(x0, x1) - lim) / std::fabs(x1 - x0);
                 };
                 coarse += above(a0, a1, 0.999);
-                const double dA = A[k + 1] - A[k], dB = B[k + 1] - B[k];
-                wide += above(std::fabs(dA), std::fabs(dA + dB * (n - 1.0)), 1.03);
+                if (a % 4 == 0) {
+                    const double dA = A[k + 1] - A[k], dB = B[k + 1] - B[k];
+                    wide += 4.0 * above(std::fabs(dA), std::fabs(dA + dB * (n - 1.0)), 1.03);
+                }
                 pairs += 1.0;
             }
         }
         for (int k0 = 0; k0 < g.Nu; k0 += 32) {
             const int kend = std::min(k0 + 32, g.Nu);
-            CellCtaGeo c;
+            CellCtaGeo c{};
             c.bAk0 = A[k0]; c.bBk0 = B[k0]; c.bAke = A[kend]; c.bBke = B[kend];
             c.Qmin = 1e300; c.Qmax = -1e300;
             for (int k = k0; k < kend; ++k) { c.Qmin = std::min(c.Qmin, Q[k]); c.Qmax = std::max(c.Qmax, Q[k]); }
-            for (int sh = 0; sh < 3; ++sh) {
-                const int RG = shapes[sh][0] * shapes[sh][1];
-                for (int rg0 = 0; rg0 < g.Nv; rg0 += RG) {
-                    c.zlo = zd0 + rg0 * dvv;
-                    c.zhi = zd0 + (rg0 + RG) * dvv;
-                    for (int L : {0, h.nlines - 1}) {
-                        const CellWindow w = cell_window(c, h, L, z0dz, h.npix, g.D, 1 << 30, 1 << 30);
-                        if (w.empty) continue;
-                        const double ph = std::fma(c.bBke, (double)L, c.bAke);
-                        const int phi = std::min((int)std::ceil(ph) - 1, h.npix - 1);
-                        maxspan = std::max(maxspan, phi - w.p0 + 1);
-                        maxnz[sh] = std::max(maxnz[sh], (double)(w.zlast - w.z0 + 1));
-                    }
-                }
-            }
+            blocks.push_back(c);
         }
+        views.push_back(h);
     }
     const bool fine = pairs > 0.0 && coarse < 0.05 * pairs;
     // a column of width w pixels overlaps three with probability w - 1: above
@@ -291,15 +279,51 @@ CellPlans plan_cell_shapes(const Geom& g, int cap_z) {
     // runs twice (us for 2 / 3 pixels a pass: 12 % of the lines 5829 / 6385,
     // 22 % 5140 / 5245, 64 % 1033 / 877, 82 % 1463 / 1083)
     const int nb = wide > 0.3 * pairs ? 3 : 2;
-    auto make = [&](int sh) {
-        CellPlan p{false, round_up(std::max(maxspan, 8), 8), std::min((int)maxnz[sh], cap_z), shapes[sh][0], shapes[sh][1], fine, nb};
+    // Plan of one launch shape: the largest of cell_window's windows over the
+    // sampled views' CTAs (its pixel part once per block and line, its slices per
+    // row group; called for the default shape and for the one launched)
+    auto make = [&](int R, int NW) {
+        const int RG = R * NW;
+        auto ifloor = [](double x) { const int i = (int)x; return i - (x < (double)i); };  // |x| < 1e8
+        int span = 0, nz = 0;
+        for (size_t a = 0; a < views.size(); ++a) {
+            const ViewHdr& h = views[a];
+            for (int kb = 0; kb < nblk; ++kb) {
+                const CellCtaGeo& c = blocks[a * nblk + kb];
+                for (int L : {0, h.nlines - 1}) {
+                    const double pl = std::fma(c.bBk0, (double)L, c.bAk0), ph = std::fma(c.bBke, (double)L, c.bAke);
+                    const double q = std::fma(h.q1, (double)L, h.q0), g0 = c.Qmin * q, g1 = c.Qmax * q;
+                    const bool in = pl > -1.0e8 && ph < 1.0e8;
+                    const int plo = in ? std::max(ifloor(pl), 0) : 0;
+                    const int phi = std::min((int)std::ceil(ph) - 1, h.npix - 1);
+                    for (int rg0 = 0; rg0 < g.Nv; rg0 += RG) {
+                        const double zlo = zd0 + rg0 * dvv, zhi = zd0 + (rg0 + RG) * dvv;
+                        const double a0 = g0 * zlo, a1 = g1 * zlo, b0 = g0 * zhi, b1 = g1 * zhi;
+                        const double tl = std::min(std::min(a0, a1), std::min(b0, b1)) - z0dz;
+                        const double th = std::max(std::max(a0, a1), std::max(b0, b1)) - z0dz;
+                        int z0 = 0, zlast = 0;
+                        const bool ok = in && tl > -1.0e8 && th < 1.0e8;
+                        if (ok) {
+                            z0 = std::max(ifloor(tl) - 1, -1);
+                            zlast = std::min(ifloor(th) + 1, g.D);
+                            if (plo > phi || z0 > zlast) continue;
+                        }
+                        span = std::max(span, phi - (ok ? plo & ~7 : 0) + 1);
+                        nz = std::max(nz, zlast - z0 + 1);
+                    }
+                }
+            }
+        }
+        CellPlan p{false, round_up(std::max(span, 8), 8), std::min(nz, cap_z), R, NW, fine, nb};
         p.ok = p.BP <= 256 && p.BZ <= 256 && p.BZ >= 1 &&
                (size_t)CELL_NS * p.BP * (p.BZ + 1) * 4 + (size_t)std::max(g.W, g.H) * 16 + 8 * CELL_NS <= 200 * 1024;
         return p;
     };
     CellPlans r;
-    r.base = make(0);
-    r.launch = make(fine ? 2 : 1);
+    r.base = make(cell_rows_per_thread(g), CELL_NW);
+    int R = r.base.R, NW = r.base.NW;
+    cell_shape(g.Nv, fine, R, NW);
+    r.launch = R == r.base.R && NW == r.base.NW ? r.base : make(R, NW);
     // the default shape where the other's windows leave an SM fewer warps (its
     // registers allow 16)
     auto warps = [&](const CellPlan& p) {
