@@ -69,3 +69,22 @@ def test_noalloc_rejects_oversized_requests(cuda):
     assert "fixed" in L.xr_last_error().decode()
     torch.cuda.synchronize()
     assert torch.count_nonzero(out).item() == 0
+
+
+def test_noalloc_takes_what_fills_its_scratch(cuda):
+    """The largest request of one image (A) that fits: 128 bytes a view, 16 a boundary and 28 a cell, rounded up to 256
+    in each of the seven tables, and the image's transpose (rows padded to eight)."""
+    geom = _geom(1)
+    up = lambda n: (n + 255) // 256 * 256  # noqa: E731
+
+    def need(V):
+        return up(128 * V) + 2 * up(8 * V * (geom.Nu + 1)) + 2 * up(8 * V * geom.Nu) + 3 * up(4 * V * geom.Nu) + \
+            up(4 * geom.W * ((geom.H + 7) // 8 * 8))
+    V = 4000
+    while need(V + 1) <= SCRATCH_BYTES:
+        V += 1
+    ang = torch.linspace(0.0, 2.0 * math.pi, V + 1)[:-1].add(0.01).to(cuda)
+    img = torch.rand(1, 1, geom.H, geom.W, generator=torch.Generator().manual_seed(8)).to(cuda)
+    want = _native.apply(2, "A", img, geom, ang)
+    got = _noalloc("A", img, geom, ang, torch.full_like(want, float("nan")))
+    assert float((got - want).norm() / want.norm()) < 1e-6

@@ -621,7 +621,7 @@ PfxStagePlan plan_pfx_stage(const Geom& g) {
                     double slack = 0.0;
                     if (g.type == GEO_ARC) {
                         const double wd = (double)(kw1 - kw0 + 1) * g.du;
-                        slack = 1.01 * g.dz * g.sdd / std::fabs(h.sperp) * wd * wd / 8.0 + 1e-12;
+                        slack = 1.01 * g.dz * g.sdd / std::fabs(h.sperp()) * wd * wd / 8.0 + 1e-12;
                     }
                     const double Rlo = std::min(colR(kw0), colR(kw1)) - slack, Rhi = std::max(colR(kw0), colR(kw1)) + slack;
                     if (!(d0 > 0.0 && d1 > 0.0 && Rlo > 0.0)) { bad = true; continue; }

@@ -80,10 +80,13 @@ struct alignas(16) ViewHdr {
     double q0, q1;          // 1 / Mv(L) = q0 + q1 * L   (1 for parallel)
     double beta, s, c;
     double sx, sy;          // source
-    double spar, sperp;     // source coordinate along / across the axis
     double perpA, perpB;    // perpendicular coordinate of line L = perpA + perpB * L
     double dpix;            // pixel size along the line (dx or dy)
+    // source coordinate along / across the axis
+    __host__ __device__ double spar() const { return use_x ? sx : sy; }
+    __host__ __device__ double sperp() const { return use_x ? sy : sx; }
 };
+static_assert(sizeof(ViewHdr) == 128, "the fixed scratch of xr_dd2d_noalloc is counted in headers of 128 bytes");
 
 // Per-view tables, structure of arrays, view-major.
 //   pos_k(L) = bA[k] + bB[k] * L : position of detector boundary k (traversal
@@ -208,14 +211,12 @@ __host__ __device__ inline void make_view_hdr(const Geom& g, float ang, ViewHdr&
     h.cf = (float)h.c;
     h.sxr = (float)h.sx;
     h.syr = (float)h.sy;
-    h.spar = h.use_x ? h.sx : h.sy;
-    h.sperp = h.use_x ? h.sy : h.sx;
     h.nlines = h.use_x ? g.H : g.W;
     h.npix = h.use_x ? g.W : g.H;
     if (h.use_x) { h.perpA = (0.5 * g.H - 0.5) * g.dy + g.shy; h.perpB = -g.dy; }
     else         { h.perpA = (0.5 - 0.5 * g.W) * g.dx + g.shx; h.perpB = g.dx; }
     if (g.type == GEO_PARALLEL) { h.q0 = 1.0; h.q1 = 0.0; }
-    else { h.q0 = 1.0 - h.perpA / h.sperp; h.q1 = -h.perpB / h.sperp; }
+    else { h.q0 = 1.0 - h.perpA / h.sperp(); h.q1 = -h.perpB / h.sperp(); }
     h.dpix = h.use_x ? g.dx : g.dy;
     h.dcx = (float)sin(h.beta + g.shu);
     h.dcy = (float)(-cos(h.beta + g.shu));

@@ -137,8 +137,8 @@ __device__ __forceinline__ void setup_view_entry(const Geom& g, const int dim3d,
         vt.colM[oc] = 0.0f;
         return;
     }
-    const double aa = 0.5 * (Dk + Dk1) - h.spar;
-    const double F = aa * aa + h.sperp * h.sperp;
+    const double aa = 0.5 * (Dk + Dk1) - h.spar();
+    const double F = aa * aa + h.sperp() * h.sperp();
     double M = 1.0;
     if (dim3d) {
         if (arcf) {
@@ -151,12 +151,12 @@ __device__ __forceinline__ void setup_view_entry(const Geom& g, const int dim3d,
         }
         // s_A = dperp / (area * triangle_cosine): forward3d.cpp:331-343.
         const double rs = (g.type == GEO_FLAT) ? g.sod / g.sdd : 1.0;
-        put(M / g.dz, g.dz / M, (float)(dperp / (fabs(h.sperp) * (Dk1 - Dk) * M * g.dv * rs)));
+        put(M / g.dz, g.dz / M, (float)(dperp / (fabs(h.sperp()) * (Dk1 - Dk) * M * g.dv * rs)));
         vt.colF[oc] = (float)F;
         vt.colM[oc] = (float)M;
     } else {
         // 2D: dperp / ((D1 - D0) * cos_weight), system_matrix2d.cpp:213,251.
-        put(M / g.dz, g.dz / M, (float)(dperp * sqrt(F) / (fabs(h.sperp) * (Dk1 - Dk))));
+        put(M / g.dz, g.dz / M, (float)(dperp * sqrt(F) / (fabs(h.sperp()) * (Dk1 - Dk))));
         vt.colF[oc] = 1.0f;
         vt.colM[oc] = 0.0f;
     }

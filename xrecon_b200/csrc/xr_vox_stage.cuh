@@ -152,7 +152,7 @@ __device__ inline int4 pfx_window(const Geom& g, const GeomF& gf, const ViewTabl
     if (g.type == GEO_ARC) {
         // colR = dz (1 -/+ sdd trig(angle) / sperp): amplitude dz sdd / |sperp|
         const double wd = (double)(kw1 - kw0 + 1) * du;
-        slack = 1.01 * g.dz * g.sdd / fabs(h.sperp) * wd * wd / 8.0 + 1e-12;
+        slack = 1.01 * g.dz * g.sdd / fabs(h.sperp()) * wd * wd / 8.0 + 1e-12;
     }
     const double Rlo = fmin(Ra, Rb) - slack, Rhi = fmax(Ra, Rb) + slack;
     if (!(d0 > 0.0 && d1 > 0.0 && Rlo > 0.0)) return unfit;
