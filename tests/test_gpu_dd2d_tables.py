@@ -194,3 +194,24 @@ def test_columns_finer_than_the_guess(cuda, du, n, x, B):
         ok = np.isfinite(want)
         got = _run(op, sino, opts, ang, cuda).cpu().numpy()
         assert rel_l2(got[ok], want[ok]) < 1e-5, op
+
+
+def test_ragged_tables_are_capped(cuda):
+    """An image whose line tables alone are past the cap of a batch's tables (1 GiB) is walked, beside one that has
+    tables; both agree with the single-scan calls (two FP32 orders of summation: 1e-5)."""
+    from xrecon_b200 import geometry as G
+    from xrecon_b200.projector import Projector2d
+    from xrecon_b200.ragged import RaggedFBP2d
+    P = [Projector2d(G.Volume2d((n, n - 3), 300.0 / n), G.FanBeam2d(G.Detector2d(90, 8.0), 500.0, 1000.0, "arc")).to(cuda)
+         for n in (8200, 64)]
+    ang = [torch.arange(V) * (2 * math.pi / V) + 0.05 for V in (2, 9)]
+    plan = RaggedFBP2d(P, ang, autotune=False, graph=False)
+    assert plan.workspace.numel() < 1 << 30
+    gen = torch.Generator(device=cuda).manual_seed(9)
+    img = [torch.rand(1, 1, n - 3, n, generator=gen, device=cuda) for n in (8200, 64)]
+    sino, recon = plan(img)
+    for i in range(2):
+        want = P[i].projection(img[i], ang[i].to(cuda))
+        assert float((sino[i] - want).norm() / want.norm()) < 1e-5
+        want = P[i].filtered_backprojection(sino[i], ang[i].to(cuda))
+        assert float((recon[i] - want).norm() / want.norm()) < 1e-5

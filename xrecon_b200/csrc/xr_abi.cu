@@ -1788,6 +1788,16 @@ int xr_ragged2d_plan_create(const xr_ragged2d_instance* inst, int ninst, xr_ragg
     RaggedLayout& L = P->lay;
     L.desc = o; o = align256(o + (size_t)ninst * sizeof(RaggedDev));
     L.sync = o; o = align256(o + 64);
+    // Line and row tables up to IL_GROUP_MAX in all (as of a single scan); what
+    // no longer fits is walked (offset 0: no table).
+    size_t tables = 0;
+    auto reserve = [&](std::vector<size_t>& at, std::vector<size_t>& flags, size_t bytes, size_t flag_bytes) {
+        const bool fits = tables + bytes <= IL_GROUP_MAX;
+        at.push_back(fits ? o : 0);
+        if (fits) tables += bytes, o = align256(o + bytes);
+        flags.push_back(o);
+        o = align256(o + flag_bytes);
+    };
     long long tot[10] = {0};
     for (int i = 0; i < ninst; ++i) {
         const Geom g = geom_from(&inst[i].geom);
@@ -1813,11 +1823,9 @@ int xr_ragged2d_plan_create(const xr_ragged2d_instance* inst, int ninst, xr_ragg
         L.colM.push_back(o); o = align256(o + Vs * g.Nu * sizeof(float));
         L.arc.push_back(o);
         if (g.type == GEO_ARC) o = align256(o + 2 * Vs * (g.Nu + 1) * sizeof(float4));  // Bw's chained walks
-        L.lines.push_back(o); o = align256(o + line_table_entries(g.W, g.H) * sizeof(double2));
-        L.lflags.push_back(o); o = align256(o + (size_t)(g.W + g.H) * sizeof(int));
         L.filt.push_back(o); o = align256(o + Vs * g.Nu * sizeof(float));
-        L.tab.push_back(o);  o = align256(o + Vs * (g.Nu + 2) * ROW_ENTRY_BYTES + 512);
-        L.flags.push_back(o); o = align256(o + Vs * sizeof(float));
+        reserve(L.lines, L.lflags, line_table_entries(g.W, g.H) * sizeof(double2), (size_t)(g.W + g.H) * sizeof(int));
+        reserve(L.tab, L.flags, Vs * (g.Nu + 2) * ROW_ENTRY_BYTES + 512, Vs * sizeof(float));
     }
     for (int l = 0; l < 10; ++l) {
         if (tot[l] > 0x7fffffffll) { delete P; return fail(XR_ERR_UNSUPPORTED, "ragged batch too large"); }
@@ -1872,10 +1880,12 @@ int xr_ragged2d_plan_bind(xr_ragged2d_plan* P, const float* images, float* sino,
         r.cw = column_width(r.g, 0);
         r.scale = in.scale;
         r.img = images + in.img_offset;
-        r.lines = LineTable{reinterpret_cast<double2*>(ws + L.lines[i]), reinterpret_cast<int*>(ws + L.lflags[i]), r.g.W, r.g.H};
+        r.lines = LineTable{L.lines[i] ? reinterpret_cast<double2*>(ws + L.lines[i]) : nullptr,
+                            reinterpret_cast<int*>(ws + L.lflags[i]), r.g.W, r.g.H};
         r.sino = sino + in.sino_offset;
         r.filt_out = reinterpret_cast<float*>(ws + L.filt[i]);
         r.tab = row_table_at(ws + L.tab[i], (size_t)in.nview * (r.g.Nu + 2));
+        if (!L.tab[i]) r.tab.q = nullptr;
         r.eps = reinterpret_cast<float*>(ws + L.flags[i]);
         r.recon = recon + in.img_offset;
         r.ang = angles + in.ang_offset;

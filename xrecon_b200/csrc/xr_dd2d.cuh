@@ -371,7 +371,7 @@ struct Spread {
 };
 
 struct LineTable {
-    double2* q;  // H lines of W + 2, then W lines of H + 2
+    double2* q;  // H lines of W + 2, then W lines of H + 2; null: no table, every line is flagged
     int* flags;  // H, then W
     int W, H;
     __host__ __device__ __forceinline__ size_t start(bool rows, int L) const {
@@ -463,9 +463,9 @@ __device__ __forceinline__ void cell2t_walk(const Geom2F& f, const ViewTables& v
     const double q0 = h.q0, q1 = h.q1;
     const float dpixf = (float)h.dpix;
     const int* flags = tab.flags + (rows ? 0 : tab.H);
-    // columns whose boundaries are not in order on every line are walked: a
-    // ray past 90 degrees from the axis, or an image with lines behind the
-    // source's plane, which a column overlaps nowhere
+    // columns whose boundaries are not in order on every line are walked: a ray
+    // past 90 degrees from the axis, or an image with lines behind the source's
+    // plane, which a column overlaps nowhere
     const double nl = (double)(nlines - 1);
     bool ordered = true;
 #pragma unroll
@@ -475,7 +475,7 @@ __device__ __forceinline__ void cell2t_walk(const Geom2F& f, const ViewTables& v
         const double dL = (double)L;
         float lf = cw;
         if (MODE == OP_A) lf = dpixf * rcp_fast((float)fma(q1, dL, q0));
-        if (flags[L] || !ordered) {
+        if (!ordered || flags[L]) {
             if (!(fma(q1, dL, q0) > 0.0)) continue;
             const double p0 = fma(B[0], dL, A[0]), p1 = fma(B[1], dL, A[1]), p2 = fma(B[2], dL, A[2]);
             acc[0] += line_walk(tab, img, rows, L, npix, p0, p1, lf);

@@ -44,7 +44,8 @@ struct RaggedDev {
     LineTable lines;
     float* sino;
     float* filt_out;
-    RowTable tab;   // row tables of filt_out and their error bounds (xr_dd2d.cuh)
+    RowTable tab;   // row tables of filt_out and their error bounds (xr_dd2d.cuh; q null: no
+                    // tables, every row is walked)
     float* eps;
     float* recon;
     const float* ang;
@@ -138,7 +139,10 @@ ragged2d_fbp_kernel(const RaggedDev* __restrict__ inst, const int ninst, const i
             for (int k = tid; k <= g.Nu; k += blockDim.x) setup_view_entry(g, 0, I.ang[lt], lt, k, I.vt, g.type == GEO_ARC);
         } else {
             const int l = (lt - I.nview) * 8 + (tid >> 5);
-            if (l < g.W + g.H) build_line_table(I.img, I.lines, l, tid & 31);
+            if (l < g.W + g.H) {
+                if (I.lines.q) build_line_table(I.img, I.lines, l, tid & 31);
+                else I.lines.flags[l] = 1;
+            }
         }
     }
     if (!grid_barrier(bar, nb)) return;
@@ -193,6 +197,10 @@ ragged2d_fbp_kernel(const RaggedDev* __restrict__ inst, const int ninst, const i
             }
             if (j < Nu) a0 = fmaf(x[j], fi[j], a0);
             I.filt_out[(size_t)v * Nu + i] = a0 + a1;
+        }
+        if (!I.tab.q) {  // uniform over the CTA
+            if (tid == 0) I.eps[v] = ROW_WALK;
+            continue;
         }
         __syncthreads();  // the whole row is in filt_out
         const float* y = I.filt_out + (size_t)v * Nu;
