@@ -66,6 +66,10 @@ typedef struct {
 /* Device workspace (bytes) that xr_dd2d / xr_dd3d need for these arguments,
  * for any storage dtype. */
 size_t xr_dd2d_workspace_size(int op, const xr_geom2d* geom, int nbatch, int nview);
+/* The least that xr_dd2d takes: without the row and line tables (1 GiB at most)
+ * or the interleaved batch, whose results a smaller workspace gives one image at
+ * a time, pixel by pixel and the same to float32 rounding. */
+size_t xr_dd2d_workspace_min(int op, const xr_geom2d* geom, int nbatch, int nview);
 size_t xr_dd3d_workspace_size(int op, const xr_geom3d* geom, int nbatch, int nview);
 
 /*
@@ -205,13 +209,14 @@ int xr_set_plain_kernels(int on);
  * device allocator.  For such callers a cudaMalloc in mid-run can fail, or
  * stall the device while it waits for free memory.
  *
- * Same operators, layouts and results as xr_dd2d.  The caller still passes
+ * Same operators and layouts as xr_dd2d, and the same results as it gives in a
+ * workspace of that size (see xr_dd2d_workspace_min).  The caller still passes
  * its inputs and outputs; the scratch (per-view tables and the flipped image
  * transpose) lives in a fixed static device array of
  * XR_NOALLOC_SCRATCH_BYTES inside the library, held by every GPU that loads
  * the library until the process exits.  No call allocates or frees device
  * memory.  Requests that need more scratch than that (see
- * xr_dd2d_workspace_size) fail with XR_ERR_WORKSPACE.  Every scratch byte a
+ * xr_dd2d_workspace_min) fail with XR_ERR_WORKSPACE.  Every scratch byte a
  * call reads is first written by the same call, so nothing needs clearing.
  * The first call on a device looks up the array's device address
  * (cudaGetSymbolAddress) and caches it per device and CUDA context (after a

@@ -215,3 +215,41 @@ def test_ragged_tables_are_capped(cuda):
         assert float((sino[i] - want).norm() / want.norm()) < 1e-5
         want = P[i].filtered_backprojection(sino[i], ang[i].to(cuda))
         assert float((recon[i] - want).norm() / want.norm()) < 1e-5
+
+
+@pytest.mark.parametrize("op,B", [("A", 1), ("BT", 1), ("B", 1), ("AT", 3), ("A", 8), ("BW", 8)])
+def test_without_memory_for_the_tables(cuda, monkeypatch, op, B):
+    """Where the device has no room for the tables or the interleaved batch, the call goes without: the same to
+    float32 rounding (1e-5 relative L2, two orders of summation)."""
+    import ctypes
+
+    from xrecon_b200 import _native
+    from xrecon_b200.backend import HostGeometry
+    opts = _opts("flat", 130, 121, 200, 1.8)
+    geom = HostGeometry(2, opts.tolist()).struct
+    ang = (np.arange(50) * 0.13).astype(np.float32)
+    shape = (B, 1, 121, 130) if op in IMAGE_IN else (B, 1, 50, 200)
+    x = np.random.default_rng(10).random(shape).astype(np.float32)
+    want = _run(op, x, opts, ang, cuda)
+    least = _native.lib().xr_dd2d_workspace_min(_native.OPS[op], ctypes.byref(geom), B, 50)
+    room = _native._workspace
+
+    def short(nbytes, device):
+        if nbytes > least:
+            raise torch.cuda.OutOfMemoryError("no room")
+        return room(nbytes, device)
+    monkeypatch.setattr(_native, "_workspace", short)
+    got = _run(op, x, opts, ang, cuda)
+    assert float((got - want).norm() / want.norm()) < 1e-5
+
+
+def test_line_tables_take_the_place_of_the_transpose(cuda):
+    """Host only: scratch of one large image's projection, view tables and line tables but no transpose."""
+    import ctypes
+
+    from xrecon_b200 import _native
+    from xrecon_b200.backend import HostGeometry
+    geom = HostGeometry(2, _opts("flat", 4096, 4096, 64, 90.0, 3000.0, 6000.0).tolist()).struct
+    lines = 2 * 4096 * 4098 * 16
+    size = _native.lib().xr_dd2d_workspace_size(_native.OPS["A"], ctypes.byref(geom), 1, 1)
+    assert size < lines + (1 << 20)

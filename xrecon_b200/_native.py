@@ -58,6 +58,8 @@ def lib():
     L = ctypes.CDLL(str(path))
     L.xr_dd2d_workspace_size.restype = c_size_t
     L.xr_dd2d_workspace_size.argtypes = [c_int, ctypes.POINTER(Geom2d), c_int, c_int]
+    L.xr_dd2d_workspace_min.restype = c_size_t
+    L.xr_dd2d_workspace_min.argtypes = [c_int, ctypes.POINTER(Geom2d), c_int, c_int]
     L.xr_dd3d_workspace_size.restype = c_size_t
     L.xr_dd3d_workspace_size.argtypes = [c_int, ctypes.POINTER(Geom3d), c_int, c_int]
     common = [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_size_t, c_void_p]
@@ -203,7 +205,13 @@ def apply(dim: int, op: str, x: torch.Tensor, geom, angles: torch.Tensor,
         else:
             nbytes = L.xr_dd3d_workspace_size(OPS[op], ctypes.byref(geom), nbatch, V)
             fn = L.xr_dd3d
-        ws = _workspace(nbytes, dev)
+        try:
+            ws = _workspace(nbytes, dev)
+        except torch.cuda.OutOfMemoryError:
+            least = L.xr_dd2d_workspace_min(OPS[op], ctypes.byref(geom), nbatch, V) if dim == 2 else nbytes
+            if least >= nbytes:
+                raise
+            ws = _workspace(least, dev)  # without tables: slower, the same to rounding
         stream = torch.cuda.current_stream(dev).cuda_stream
         rc = fn(OPS[op], ctypes.byref(geom), x.data_ptr(), DTYPES[x.dtype], out.data_ptr(), DTYPES[odt],
                 ang.data_ptr(), nbatch, V, ws.data_ptr(), ws.numel(), stream)

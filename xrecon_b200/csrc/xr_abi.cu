@@ -446,9 +446,10 @@ Layout layout(int dim3d, int op, const Geom& g, int nbatch, int nview, int dtype
         // line tables (B^T on the arc detector chains its angles, Bw^T weighs
         // every pixel: both walk)
         const size_t bytes = line_table_entries(g.W, g.H) * sizeof(double2);
-        if (bytes <= IL_GROUP_MAX) {
-            l.tab = o;    o = align256(o + bytes);
-            l.flags = o;  o = align256(o + (size_t)(g.W + g.H) * sizeof(int));
+        if (bytes <= IL_GROUP_MAX) {  // in the transpose's place, which only the walk reads
+            l.tab = l.volT;
+            l.flags = align256(l.tab + bytes);
+            o = std::max(o, align256(l.flags + (size_t)(g.W + g.H) * sizeof(int)));
         }
     } else if (!dim3d && op >= 0 && nbatch > 1 && nview > 0) {
         const int nb = interleave_nb(nbatch), groups = (nbatch + nb - 1) / nb;
@@ -1507,6 +1508,12 @@ size_t xr_dd2d_workspace_size(int op, const xr_geom2d* geom, int nbatch, int nvi
     if (!geom) return 0;
     const xr::Geom g = xr::geom_from(geom);
     return xr::layout(0, op, g, nbatch, nview, xr::DT_F32).total;
+}
+
+size_t xr_dd2d_workspace_min(int op, const xr_geom2d* geom, int nbatch, int nview) {
+    if (!geom) return 0;
+    const xr::Geom g = xr::geom_from(geom);
+    return xr::layout(0, op, g, nbatch, nview, xr::DT_F32).base;
 }
 
 size_t xr_dd3d_workspace_size(int op, const xr_geom3d* geom, int nbatch, int nview) {
