@@ -942,8 +942,9 @@ int run3d(int op, const Geom& g, const TI* in, TO* out, const float* ang, int nb
     dim3 block(32, VOX_NW);
     const GeomF gf = make_geomf(g, 1);
     const float atconst = (float)(g.dx * g.dy * g.dz / (g.du * g.dv));
-    // the prefix kernel addresses one view's table with 32-bit byte offsets
-    const bool prefix_ok = (double)(g.Nv + 2) * tab_pitch(g.Nu) * sizeof(float2) < 2147483648.0;
+    // one view's table is addressed with unsigned 32-bit byte offsets (a padding
+    // column more of an odd count leaves them below 2^32)
+    const bool prefix_ok = (double)(g.Nv + 2) * g.Nu * sizeof(float2) < 2147483648.0;
     if (!g_force_plain && prefix_ok) {
         float2* tab = reinterpret_cast<float2*>(ws + l.sinoS);
         const int nbv = nbatch * nview;
@@ -1292,7 +1293,7 @@ int helical(int op, const Geom& g, const HelOpts& o, const float* in, float* out
         }
         return XR_OK;
     }
-    if ((double)(g.Nv + 2) * tab_pitch(g.Nu) * sizeof(float2) >= 2147483648.0)
+    if ((double)(g.Nv + 2) * g.Nu * sizeof(float2) >= 2147483648.0)
         return fail(XR_ERR_UNSUPPORTED, "detector of %d x %d cells too large for one view's row table", g.Nu, g.Nv);
     HelZ* zw = reinterpret_cast<HelZ*>(ws + hl.zw);
     HelScanF* scan = reinterpret_cast<HelScanF*>(ws + hl.scan);
