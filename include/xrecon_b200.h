@@ -188,12 +188,23 @@ int xr_test_hooks(unsigned int hooks);
  * than a voxel) is chosen. */
 int xr_cell_plan(const xr_geom3d* geom, int* ok, int* box_pixels, int* box_z, int* rows_per_thread, int* fine);
 
+/* The launch shape of that kernel for this geometry: detector rows a thread, warps
+ * a CTA, and pixels of a column a pass of the fine walk; zeros when the line windows
+ * are not used.  Host-only. */
+int xr_cell_launch_plan(const xr_geom3d* geom, int* rows_per_thread, int* warps, int* pixels);
+
 /* Staging plan of the 3D prefix backprojection (B, Bw, A^T) for this
  * geometry: whether each view's table footprint is staged into shared memory
  * as it is (flat, parallel and arc detectors with an even column count; odd
  * counts are staged through tables padded by a column and reported as not ok),
  * and the box size in table columns x rows.  Host-only; no device is touched. */
 int xr_pfx_stage_plan(const xr_geom3d* geom, int* ok, int* box_cols, int* box_rows);
+
+/* What runs for a call of nbatch volumes and nview views: whether the tables are
+ * staged (odd column counts too), and the CTAs that share a tile's views (1: no
+ * split).  The split decides the order of the sums, so the bits of a result depend
+ * on the batch and the number of views.  Host-only. */
+int xr_pfx_launch_plan(const xr_geom3d* geom, int nbatch, int nview, int* staged, int* split);
 
 /* Testing aid: nonzero routes every operator through the plain (non-TMA)
  * kernels, so both paths can be compared. */

@@ -79,6 +79,10 @@ def lib():
     L.xr_device_error.argtypes = [ctypes.POINTER(ctypes.c_uint), c_int]
     L.xr_cell_plan.restype = c_int
     L.xr_cell_plan.argtypes = [ctypes.POINTER(Geom3d)] + [ctypes.POINTER(c_int)] * 5
+    L.xr_cell_launch_plan.restype = c_int
+    L.xr_cell_launch_plan.argtypes = [ctypes.POINTER(Geom3d)] + [ctypes.POINTER(c_int)] * 3
+    L.xr_pfx_launch_plan.restype = c_int
+    L.xr_pfx_launch_plan.argtypes = [ctypes.POINTER(Geom3d), c_int, c_int] + [ctypes.POINTER(c_int)] * 2
     L.xr_pfx_stage_plan.restype = c_int
     L.xr_pfx_stage_plan.argtypes = [ctypes.POINTER(Geom3d)] + [ctypes.POINTER(c_int)] * 3
     L.xr_set_plain_kernels.restype = c_int
@@ -401,6 +405,25 @@ def cell_plan(geom: Geom3d) -> dict:
         _raise(rc, "xr_cell_plan")
     return dict(ok=bool(vals[0].value), box_pixels=vals[1].value, box_z=vals[2].value,
                 rows_per_thread=vals[3].value, fine=bool(vals[4].value))
+
+
+def cell_launch_plan(geom: Geom3d) -> dict:
+    """Launch shape of the 3D projection kernel for a geometry (zeros: not staged)."""
+    vals = [c_int(0) for _ in range(3)]
+    rc = lib().xr_cell_launch_plan(ctypes.byref(geom), *[ctypes.byref(v) for v in vals])
+    if rc != 0:
+        _raise(rc, "xr_cell_launch_plan")
+    return dict(rows_per_thread=vals[0].value, warps=vals[1].value, pixels=vals[2].value)
+
+
+def pfx_launch_plan(geom: Geom3d, nbatch: int, nview: int) -> dict:
+    """What the 3D prefix backprojection runs for a call: staged tables, and the
+    CTAs that share a tile's views."""
+    vals = [c_int(0) for _ in range(2)]
+    rc = lib().xr_pfx_launch_plan(ctypes.byref(geom), nbatch, nview, *[ctypes.byref(v) for v in vals])
+    if rc != 0:
+        _raise(rc, "xr_pfx_launch_plan")
+    return dict(staged=bool(vals[0].value), split=vals[1].value)
 
 
 def pfx_stage_plan(geom: Geom3d) -> dict:

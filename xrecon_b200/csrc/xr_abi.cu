@@ -1626,6 +1626,27 @@ int xr_cell_plan(const xr_geom3d* geom, int* ok, int* box_pixels, int* box_z, in
     return XR_OK;
 }
 
+int xr_cell_launch_plan(const xr_geom3d* geom, int* rows_per_thread, int* warps, int* pixels) {
+    if (!geom || !rows_per_thread || !warps || !pixels) return xr::fail(XR_ERR_INVALID_ARGUMENT, "null pointer");
+    const xr::Geom g = xr::geom_from(geom);
+    if (int rc = xr::validate(g, 1, 0, 1, 1)) return rc;
+    const xr::CellPlans p = xr::plan_cell_shapes(g, 1 << 30);
+    *rows_per_thread = p.base.ok ? p.launch.R : 0;
+    *warps = p.base.ok ? p.launch.NW : 0;
+    *pixels = p.base.ok ? (p.launch.fine ? p.launch.NB : 2) : 0;
+    return XR_OK;
+}
+
+int xr_pfx_launch_plan(const xr_geom3d* geom, int nbatch, int nview, int* staged, int* split) {
+    if (!geom || !staged || !split) return xr::fail(XR_ERR_INVALID_ARGUMENT, "null pointer");
+    const xr::Geom g = xr::geom_from(geom);
+    if (int rc = xr::validate(g, 1, 0, nbatch, nview)) return rc;
+    const xr::PfxStagePlan p = xr::plan_pfx_stage(g);
+    *staged = p.ok;
+    *split = p.ok ? xr::pfx_split(g, nbatch, nview, (g.D + xr::PFX_R - 1) / xr::PFX_R, p.BC, p.BR) : 1;
+    return XR_OK;
+}
+
 int xr_pfx_stage_plan(const xr_geom3d* geom, int* ok, int* box_cols, int* box_rows) {
     if (!geom || !ok || !box_cols || !box_rows) return xr::fail(XR_ERR_INVALID_ARGUMENT, "null pointer");
     const xr::Geom g = xr::geom_from(geom);
