@@ -31,3 +31,23 @@ def test_projection_launch_shapes_match_the_oracle(cuda, Nv, du, dv):
     for op in ("A", "BT", "BWT"):
         got = _native.apply(3, op, torch.from_numpy(img).to(cuda), geom, torch.from_numpy(ang).to(cuda))
         assert rel_l2(got.cpu().numpy(), O.dd3d(op, img, opts, ang)) < 1e-5, op
+
+
+@pytest.mark.parametrize("scan,W,D,Nu,Nv,du,dv,dz", [("parallel", 64, 40, 96, 50, 1.7, 1.7, 1.0),
+                                                     ("parallel", 64, 40, 200, 50, 0.8, 1.2, 1.0),
+                                                     ("flat", 48, 60, 64, 96, 2.0, 1.1, 0.7),
+                                                     ("flat", 64, 40, 96, 50, 1.7, 1.7, 1.0)])
+def test_rows_of_a_thread_keep_their_precision(cuda, scan, W, D, Nu, Nv, du, dv, dz):
+    """Longer runs of rows a thread must not cost precision: with eight rows a thread the projection was within
+    2.6e-7 of the oracle on these scans; a quarter to spare."""
+    from xrecon_b200 import _native
+    from xrecon_b200 import geometry as G
+    from xrecon_b200.backend import HostGeometry
+    det = G.Detector3d((Nu, Nv), (du, dv), (0.3, 0.2))
+    geo = G.ParallelBeam3d(det) if scan == "parallel" else G.ConeBeam3d(det, 200.0, 400.0, scan)
+    opts = np.array(G.pack_options3d(G.Volume3d((W, W - 3, D), (1.0, 1.0, dz), (0.4, -0.2, 0.3)), geo), np.float32)
+    ang = (np.arange(5) * (2 * np.pi / 5) + 0.21).astype(np.float32)
+    img = np.random.default_rng(3).random((1, 1, D, W - 3, W)).astype(np.float32)
+    got = _native.apply(3, "A", torch.from_numpy(img).to(cuda), HostGeometry(3, opts.tolist()).struct,
+                        torch.from_numpy(ang).to(cuda))
+    assert rel_l2(got.cpu().numpy(), O.dd3d("A", img, opts, ang)) < 3.2e-7

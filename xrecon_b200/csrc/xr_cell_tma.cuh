@@ -119,6 +119,18 @@ __device__ __noinline__ void drain_stages(uint64_t* bar, int last) {
         mbar_wait_bounded(&bar[Lp % NS], (unsigned)((Lp / NS) & 1));
 }
 
+// The walks of rows of a voxel or more place row i at f + i bf from the slice that
+// holds the run's start; every WALK_BASE rows they count anew from the slice reached
+// (f + 8 bf less its floor n, 8 bf - n being exact), since FP32 rounds a position by
+// its size.
+constexpr int WALK_BASE = 8;
+__device__ __forceinline__ void rebase_walk(float bf, float& f, float& pos, float& jn) {
+    const float n = floorf(fmaf(bf, (float)WALK_BASE, f));
+    f += fmaf(bf, (float)WALK_BASE, -n);
+    pos = f;
+    jn -= n;
+}
+
 // Walk of one column's R rows over one line from global memory, with bounds
 // checks: adds the row sums to out.  Out of line and rolled, so that it costs
 // the staged walk no registers and no code; `wz` (null: 1) weighs slice j by
@@ -128,8 +140,7 @@ __device__ __noinline__ void cell_walk_global(const TI* __restrict__ base, size_
                                               const float (&w)[NB], int np, const float* wz, int nview, int R, float* out) {
     const double jf = floor(t0);
     int j = (int)jf;
-    float pos = (float)(t0 - jf), jn = 1.0f;
-    const float f = pos;
+    float pos = (float)(t0 - jf), jn = 1.0f, f = pos;
     auto band = [&]() -> float {
         if ((unsigned)j >= (unsigned)D) return 0.0f;
         const float v = band_at<TI, NB>(base + (size_t)j * plane, w, np);
@@ -138,7 +149,8 @@ __device__ __noinline__ void cell_walk_global(const TI* __restrict__ base, size_
     float vj = band();
 #pragma unroll 1
     for (int i = 0; i < R; ++i) {
-        const float top = fmaf(bf, (float)(i + 1), f);
+        if (i && i % WALK_BASE == 0) rebase_walk(bf, f, pos, jn);
+        const float top = fmaf(bf, (float)(i % WALK_BASE + 1), f);
         float a = 0.0f;
         while (jn < top) {
             a = fmaf(jn - pos, vj, a);
@@ -383,8 +395,8 @@ cell_tma3d_kernel(const Geom g, const ViewTables vt, const __grid_constant__ CUt
                     }
                     if (win.ok && bf < 0.999f) {
                         // Rows shorter than a voxel: each row crosses at most
-                        // one voxel boundary.  In window slice coordinates
-                        // u = t - (win.z0 - j0) (staged row = floor u), row i
+                        // one voxel boundary.  In slices u = t - j0 from the
+                        // run's start (staged row = floor u + j0 - win.z0), row i
                         // spans [u_i, u_{i+1}]; with n = floor(u_{i+1}) its
                         // part below n lies in slice n - 1, the slice of the
                         // previous row's top, and the rest in slice n:
@@ -398,15 +410,19 @@ cell_tma3d_kernel(const Geom g, const ViewTables vt, const __grid_constant__ CUt
                         // offset: two FMA-pipe slots, where a conversion to
                         // int and back took two on the quarter-rate
                         // conversion pipe (44 % busy).  u is clamped to the
-                        // staged slices 0 .. win.zlast - win.z0 (slices -1
+                        // staged slices win.z0 .. win.zlast (slices -1
                         // and D of the volume arrive as zeros, and the
                         // window covers every t of the CTA otherwise).
                         const unsigned live = __activemask();
-                        float fu = (float)(t0 - (double)win.z0), fu_next = fu;
+                        // (u counts from the run's start, not from the window's,
+                        // which holds all the CTA's rows: FP32 rounds a position
+                        // by its size)
+                        const int j0 = __float2int_rd(t0f);
+                        float fu = (float)(t0 - (double)j0), fu_next = fu;
                         *(volatile float*)&s_fu[tid] = fu;
-                        const float uhi = (float)(win.zlast - win.z0) + 0.999f;
-                        const unsigned sb = (unsigned)(((size_t)s * stage_elems + XR_BOUND(pc - win.p0, 0, BP - np)) * sizeof(TI)) -
-                                            0x4B400000u * pitch_b;
+                        const float ulo = (float)(win.z0 - j0), uhi = (float)(win.zlast - j0) + 0.999f;
+                        const unsigned sb = (unsigned)(((size_t)s * stage_elems + XR_BOUND(pc - win.p0, 0, BP - np)) * sizeof(TI)) +
+                                            (unsigned)(j0 - win.z0) * pitch_b - 0x4B400000u * pitch_b;
                         auto slice_at = [&](float u, float& n) -> float {
                             const float tr = __fadd_rd(u, 12582912.0f);
                             n = tr - 12582912.0f;
@@ -416,9 +432,9 @@ cell_tma3d_kernel(const Geom g, const ViewTables vt, const __grid_constant__ CUt
 #else
                             const TI* q = reinterpret_cast<const TI*>(smem_raw + off);
 #endif
-                            return band_smem<TI, NB>(q, w, np) * slice_w(win.z0 + (__float_as_int(tr) - 0x4B400000));
+                            return band_smem<TI, NB>(q, w, np) * slice_w(j0 + (__float_as_int(tr) - 0x4B400000));
                         };
-                        float up = fminf(fmaxf(fu, 0.0f), uhi);
+                        float up = fminf(fmaxf(fu, ulo), uhi);
                         float np0;
                         float bp = slice_at(up, np0);
 #pragma unroll
@@ -431,7 +447,7 @@ cell_tma3d_kernel(const Geom g, const ViewTables vt, const __grid_constant__ CUt
                                 fu = fu_next;
                                 fu_next = *(volatile float*)&s_fu[tid];
                             }
-                            const float u1 = fminf(fmaxf(fmaf(bf, (float)(i + 1), fu), 0.0f), uhi);
+                            const float u1 = fminf(fmaxf(fmaf(bf, (float)(i + 1), fu), ulo), uhi);
                             float n;
                             const float bn = slice_at(u1, n);
                             // max(0, n - u_i) = max(n, u_i) - u_i exactly
@@ -444,7 +460,7 @@ cell_tma3d_kernel(const Geom g, const ViewTables vt, const __grid_constant__ CUt
                     } else if (!FINE && win.ok) {
                         const double jf = floor(t0);
                         const int j0 = (int)jf;
-                        const float f = (float)(t0 - jf);
+                        float f = (float)(t0 - jf);
                         float pos = f, jn = 1.0f, vj;
                         // Staged voxels win.z0 .. win.zlast; below the window a
                         // single virtual zero voxel ends at win.z0, past
@@ -465,7 +481,8 @@ cell_tma3d_kernel(const Geom g, const ViewTables vt, const __grid_constant__ CUt
                         }
 #pragma unroll
                         for (int i = 0; i < R; ++i) {
-                            const float top = fmaf(bf, (float)(i + 1), f);
+                            if (i && i % WALK_BASE == 0) rebase_walk(bf, f, pos, jn);
+                            const float top = fmaf(bf, (float)(i % WALK_BASE + 1), f);
                             float a = 0.0f;
                             while (jn < top) {
                                 a = fmaf(jn - pos, vj, a);
