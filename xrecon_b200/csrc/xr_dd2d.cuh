@@ -470,18 +470,17 @@ __device__ __forceinline__ void cell2t_walk(const Geom2F& f, const ViewTables& v
     bool ordered = true;
 #pragma unroll
     for (int c = 0; c < 2; ++c)
-        ordered = ordered && (k + c >= Nu || (A[c + 1] > A[c] && fma(B[c + 1], nl, A[c + 1]) > fma(B[c], nl, A[c])));
-    for (int L = l0; L < nlines; L += ls) {
+        ordered = ordered && (k + c >= Nu || (A[c + 1] > A[c] && A[c + 1] - A[c] < 1.0e300 &&
+                                              fma(B[c + 1], nl, A[c + 1]) > fma(B[c], nl, A[c])));
+    auto factor = [&](double dL) { return MODE == OP_A ? dpixf * rcp_fast((float)fma(q1, dL, q0)) : cw; };
+    bool rest = !ordered;  // lines left to the walk
+    for (int L = ordered ? l0 : nlines; L < nlines; L += ls) {
         const double dL = (double)L;
-        float lf = cw;
-        if (MODE == OP_A) lf = dpixf * rcp_fast((float)fma(q1, dL, q0));
-        if (!ordered || flags[L]) {
-            if (!(fma(q1, dL, q0) > 0.0)) continue;
-            const double p0 = fma(B[0], dL, A[0]), p1 = fma(B[1], dL, A[1]), p2 = fma(B[2], dL, A[2]);
-            acc[0] += line_walk(tab, img, rows, L, npix, p0, p1, lf);
-            acc[1] += line_walk(tab, img, rows, L, npix, p1, p2, lf);
+        if (flags[L]) {
+            rest = true;
             continue;
         }
+        const float lf = factor(dL);
         const double2* q = tab.q + tab.start(rows, L);
         double S[3];
 #pragma unroll
@@ -493,6 +492,15 @@ __device__ __forceinline__ void cell2t_walk(const Geom2F& f, const ViewTables& v
         }
         acc[0] = fmaf(lf, (float)(S[1] - S[0]), acc[0]);
         acc[1] = fmaf(lf, (float)(S[2] - S[1]), acc[1]);
+    }
+    // after the others, so that the loop above keeps its registers
+    for (int L = rest ? l0 : nlines; L < nlines; L += ls) {
+        const double dL = (double)L;
+        if ((ordered && !flags[L]) || !(fma(q1, dL, q0) > 0.0)) continue;
+        const double p0 = fma(B[0], dL, A[0]), p1 = fma(B[1], dL, A[1]), p2 = fma(B[2], dL, A[2]);
+        const float lf = factor(dL);
+        acc[0] += line_walk(tab, img, rows, L, npix, p0, p1, lf);
+        acc[1] += line_walk(tab, img, rows, L, npix, p1, p2, lf);
     }
 }
 
