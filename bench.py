@@ -897,12 +897,11 @@ def run_gpu_arm(args, rank: int, world: int, local_rank: int):
 
     hbm, src = peaks()
     dom_t = max(t_a, t_b)
-    dom = "cell_tma3d_kernel (projection A)" if t_a >= t_b else "vox_prefix3d_kernel (backprojection B)"
+    dom = "cell_tma3d_kernel (projection A)" if t_a >= t_b else "vox_stage3d_kernel (backprojection B)"
     # what holds the kernel below the HBM roofline, from its ncu profile
-    # (profiles/cell_tma3d_A_cone_flat_64views.md, vox_prefix3d_B_cone_flat_64views.md)
-    limiter = ("instruction issue: ~70 % issue active, 'not selected' stalls, DRAM ~3 % of peak"
+    limiter = ("instruction issue: ~77 % issue active, 'not selected' stalls, DRAM nearly idle"
                if t_a >= t_b else
-               "table-lookup latency and issue: ~67 % issue active, long-scoreboard (L1 hit) stalls, DRAM idle")
+               "instruction issue: ~81 % issue active, shared-memory lookups half bank conflicts, DRAM idle")
     wl = dict(WL, V=nv)
     achieved = algo_bytes_op(wl) / dom_t / 1e9
     traffic = None

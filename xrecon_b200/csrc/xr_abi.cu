@@ -1102,8 +1102,8 @@ int run2d(int op, const Geom& g, const TI* in, void* out, int dto, const float* 
         else table2d_kernel<TI, false><<<nview, 256, 0, st>>>(g, f, ang, nview, vt, in, nbatch, tab, eps);
         if (int rc = check_cuda("table2d")) return rc;
         // View slices: first CTAs of a cluster (a CTA's warps then share each
-        // view's table in L1) until every SM holds four, what 64 registers a
-        // thread allow (720-view FBP of 256 x 256 pixels, the whole call: 256 CTAs 290 us, 512
+        // view's table in L1) until there are three for every SM, so that the four
+        // that 64 registers a thread allow are nearly all taken (720-view FBP of 256 x 256 pixels, the whole call: 256 CTAs 290 us, 512
         // CTAs 243 us); warps of a CTA only where that leaves SMs without work.
         int CS = 1, VS = 1;
         const int n1 = pix2t_ctas(g.W, g.H, 1) * nbatch;

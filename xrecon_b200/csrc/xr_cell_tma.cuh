@@ -14,7 +14,7 @@
 // The kernel is bound by instruction issue (0.77 per cycle and scheduler; DRAM
 // nearly idle), so what pays is fewer instructions per (cell, line): with 32
 // rows a thread 18.9 lane-slots, with 16 rows 22.8.  512 x 512 x 256 voxels, 1440
-// views, 1024 x 256 cells: 151.3 -> 113.3 ms.
+// views, 1024 x 256 cells: 151.3 -> 114.9 ms.
 //
 // The window is a uniform function of the line index, evaluated identically
 // by the producer thread (for line L+2) and by every consumer (for line L):

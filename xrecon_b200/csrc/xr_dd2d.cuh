@@ -22,11 +22,15 @@
 // No atomics: every output has one owner.
 //
 // Measured on a B200, before (one thread per output, no split, no tables) and
-// now, us: FBP of 256 x 256 pixels from 720 fan-flat views 1043 -> 219 (Bw 1006
-// -> about 180, the call less its other launches); a batch of eight 512 x 512 arc slices, A + A^T over 360 views, 10825 ->
-// 1628; A + FBP of 16 ragged fan-arc instances 20344 -> 10730.  The pixel gathers
+// now, us: FBP of 256 x 256 pixels from 720 fan-flat views 1055 -> 223; a batch of
+// eight 512 x 512 arc slices, A + A^T over 360 views, 10855 -> 1546; A + FBP of 16
+// ragged fan-arc instances 20344 -> 12300.  The pixel gathers
 // are held by the latency of their table entries in L1 and by conversions, the
 // batched walks by L1 wavefronts and lanes in different columns.
+//
+// Which of these a call takes goes by the batch, the scratch given and the values
+// (a row of too wide a spread is walked), so the same image may differ by float32
+// rounding between them.
 #pragma once
 
 #include <cmath>
@@ -736,9 +740,10 @@ __host__ __device__ inline int pix2d_tiles(int W, int H) {
 // A CTA's 8 warps are 8 / VS tiles times VS view slices.  NB = 1: the
 // sinograms [batch][view][column] of type TI; NB > 1: their interleaved FP32
 // copy.  blockIdx.y is the group of NB images.
-// A^T of eight images held at 80 registers (three CTAs per SM; 126 unbound, 24
-// bytes of spills): a batch of eight 512 x 512 slices, A + A^T, 1784 -> 1675 us; B
-// and Bw got slower that way (167 -> 190, 1235 -> 1266 us) and stay unbound.
+// A^T of eight images held at 80 registers (three CTAs per SM; 126 unbound, 32
+// bytes of spills): a batch of eight 512 x 512 slices, A + A^T, 1732 -> 1628 us
+// when it came; B and Bw got slower that way (167 -> 190, 1235 -> 1266 us) and stay
+// unbound.
 template <typename TI, int NB, int MODE>
 __global__ void __launch_bounds__(256, MODE == OP_AT && NB == 8 ? 3 : 1)
 pix2d_kernel(const Geom2F f, const ViewTables vt, const TI* __restrict__ sino, void* __restrict__ img,
