@@ -882,7 +882,8 @@ __device__ __forceinline__ float build_row_table(const Geom2F& f, const ViewTabl
                 a = (double)y * dA;
                 b = (double)y * dB;
             }
-            width = fminf(width, fminf((float)dA, (float)fma(dB, nl, dA)));
+            const double d1 = fma(dB, nl, dA);
+            width = dA > 0.0 && d1 > 0.0 ? fminf(width, (float)fmin(dA, d1)) : 0.0f;
         }
         const double a0 = a, b0 = b;
 #pragma unroll
