@@ -188,10 +188,10 @@ int xr_test_hooks(unsigned int hooks);
  * than a voxel) is chosen. */
 int xr_cell_plan(const xr_geom3d* geom, int* ok, int* box_pixels, int* box_z, int* rows_per_thread, int* fine);
 
-/* The launch shape of that kernel for this geometry: detector rows a thread, warps
- * a CTA, and pixels of a column a pass of the fine walk; zeros when the line windows
- * are not used.  Host-only. */
-int xr_cell_launch_plan(const xr_geom3d* geom, int* rows_per_thread, int* warps, int* pixels);
+/* The launch shape of that kernel for a call of nbatch volumes and nview views:
+ * detector rows a thread, warps a CTA, and pixels of a column a pass of the fine
+ * walk; zeros when the line windows are not used.  Host-only. */
+int xr_cell_launch_plan(const xr_geom3d* geom, int nbatch, int nview, int* rows_per_thread, int* warps, int* pixels);
 
 /* Staging plan of the 3D prefix backprojection (B, Bw, A^T) for this
  * geometry: whether each view's table footprint is staged into shared memory

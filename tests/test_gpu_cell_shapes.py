@@ -51,3 +51,25 @@ def test_rows_of_a_thread_keep_their_precision(cuda, scan, W, D, Nu, Nv, du, dv,
     got = _native.apply(3, "A", torch.from_numpy(img).to(cuda), HostGeometry(3, opts.tolist()).struct,
                         torch.from_numpy(ang).to(cuda))
     assert rel_l2(got.cpu().numpy(), O.dd3d("A", img, opts, ang)) < 3.2e-7
+
+
+@pytest.mark.parametrize("Nv,V", [(24, 640), (64, 640), (128, 256), (160, 256)])
+@pytest.mark.parametrize("du,dv", [(1.3, 1.0), (4.4, 1.0), (1.3, 3.0)])
+def test_projection_shapes_of_large_grids_match_the_oracle(cuda, Nv, V, du, dv):
+    """As above with the views repeated until the grid takes the shapes of large scans (16 and 32 rows a thread; rows
+    of a voxel and a half, for which that is 16), and every repeat the same bits."""
+    from xrecon_b200 import _native
+    from xrecon_b200 import geometry as G
+    from xrecon_b200.backend import HostGeometry
+    D = max(4, int(Nv * 0.45 * dv))
+    geo = G.ConeBeam3d(G.Detector3d((45, Nv), (du, dv), (0.3, 0.2)), 200.0, 400.0, "flat")
+    opts = np.array(G.pack_options3d(G.Volume3d((26, 23, D), 1.0, (0.4, -0.2, 0.3)), geo), np.float32)
+    geom = HostGeometry(3, opts.tolist()).struct
+    assert _native.cell_launch_plan(geom, 1, V)["rows_per_thread"] == (16 if dv > 1.0 or Nv == 24 else 32)
+    ang = np.array([0.03, 0.7, np.pi / 4, 2.2, 3.9, 5.6, 4.4, 1.2], np.float32)
+    img = np.random.default_rng(Nv).random((1, 1, D, 23, 26)).astype(np.float32)
+    for op in ("A", "BT", "BWT"):
+        got = _native.apply(3, op, torch.from_numpy(img).to(cuda), geom, torch.from_numpy(np.tile(ang, V // 8)).to(cuda))
+        first = got[:, :, :8]
+        assert rel_l2(first.cpu().numpy(), O.dd3d(op, img, opts, ang)) < 1e-5, op
+        assert torch.equal(got.reshape(1, 1, V // 8, 8, Nv, 45), first[:, :, None].expand(1, 1, V // 8, 8, Nv, 45)), op

@@ -80,7 +80,7 @@ def lib():
     L.xr_cell_plan.restype = c_int
     L.xr_cell_plan.argtypes = [ctypes.POINTER(Geom3d)] + [ctypes.POINTER(c_int)] * 5
     L.xr_cell_launch_plan.restype = c_int
-    L.xr_cell_launch_plan.argtypes = [ctypes.POINTER(Geom3d)] + [ctypes.POINTER(c_int)] * 3
+    L.xr_cell_launch_plan.argtypes = [ctypes.POINTER(Geom3d), c_int, c_int] + [ctypes.POINTER(c_int)] * 3
     L.xr_pfx_launch_plan.restype = c_int
     L.xr_pfx_launch_plan.argtypes = [ctypes.POINTER(Geom3d), c_int, c_int] + [ctypes.POINTER(c_int)] * 2
     L.xr_pfx_stage_plan.restype = c_int
@@ -407,10 +407,10 @@ def cell_plan(geom: Geom3d) -> dict:
                 rows_per_thread=vals[3].value, fine=bool(vals[4].value))
 
 
-def cell_launch_plan(geom: Geom3d) -> dict:
-    """Launch shape of the 3D projection kernel for a geometry (zeros: not staged)."""
+def cell_launch_plan(geom: Geom3d, nbatch: int, nview: int) -> dict:
+    """Launch shape of the 3D projection kernel for a call (zeros: not staged)."""
     vals = [c_int(0) for _ in range(3)]
-    rc = lib().xr_cell_launch_plan(ctypes.byref(geom), *[ctypes.byref(v) for v in vals])
+    rc = lib().xr_cell_launch_plan(ctypes.byref(geom), nbatch, nview, *[ctypes.byref(v) for v in vals])
     if rc != 0:
         _raise(rc, "xr_cell_launch_plan")
     return dict(rows_per_thread=vals[0].value, warps=vals[1].value, pixels=vals[2].value)

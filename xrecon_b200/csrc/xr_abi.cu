@@ -9,6 +9,7 @@
 #include <cudaTypedefs.h>
 #include <nvtx3/nvToolsExt.h>
 
+#include <algorithm>
 #include <array>
 #include <atomic>
 #include <cstring>
@@ -184,14 +185,20 @@ int round_up(int v, int m) { return (v + m - 1) / m * m; }
 // of one warp waits on its own copies (us for R = 16 / 32: 64 rows 4512 / 3758,
 // 83 rows 1281 / 1083, 96 rows 6643 / 5140, 160 rows 5266 / 4971; 32 rows, one
 // warp at R = 32, 877 / 1734; eight warps of 8 or 16 rows took 5858, 1895, 9143,
-// 6888 and 1748).
-void cell_shape(int Nv, bool fine, int& R, int& NW) {
-    int best = 1 << 30;
-    for (int r = fine ? 8 : 16; r <= (fine ? 32 : 16); r *= 2) {
+// 6888 and 1748).  A grid that does not fill the GPU's 16 warps per SM gains nothing
+// from fewer warps: its time is one warp's, so it takes the fewest rows (`blocks`
+// column blocks x views x batch; us for R = 8 / 16: 24 rows, 435 blocks 95 / 144,
+// 40 rows, 400 blocks 105 / 154; 60 rows, 700 blocks, 5600 / 2800 warps 271 / 229).
+// Rows of a voxel or more take eight a thread only there.
+void cell_shape(int Nv, bool fine, double blocks, int& R, int& NW) {
+    double best = 1e300;
+    for (int r = 8; r <= (fine ? 32 : 16); r *= 2) {
         // rows of a CTA: at most 128, split evenly over the fewest CTAs
         const int groups = (Nv + 127) / 128, per = (Nv + groups - 1) / groups, nw = (per + r - 1) / r;
         if (nw > CELL_NW || (fine && nw == 1 && r > 8)) continue;
-        const int cost = groups * nw * (r + 9);
+        const double rounds = blocks * groups * nw / (148.0 * 16.0);
+        if (!fine && r == 8 && rounds > 1.0) continue;
+        const double cost = std::max(1.0, rounds) * (r + 9);
         if (cost <= best) best = cost, R = r, NW = nw;
     }
 }
@@ -204,16 +211,28 @@ size_t cell_smem(const CellPlan& p, int maxlines) {
 // evaluating the kernel's own window function over the CTAs of views sampled
 // densely in angle (the window depends on the angle only through smooth
 // functions; the 45-degree axis switches are sampled on both sides).  Cached
-// per geometry.
-CellPlans plan_cell_shapes(const Geom& g, int cap_z) {
+// per geometry, with every launch shape taken so far; `images` (views x batch)
+// decides the shape, 0: a grid that fills the GPU.
+CellPlans plan_cell_shapes(const Geom& g, int cap_z, long long images) {
+    struct Known {
+        CellPlan base;
+        std::vector<CellPlans> shapes;  // base and launch, by the launch's rows and warps as asked for
+        std::vector<std::pair<int, int>> asked;
+    };
     static std::mutex mu;
-    static std::map<std::string, CellPlans> cache;
+    static std::map<std::string, Known> cache;
+    const double grid = images > 0 ? (double)images * ((g.Nu + 31) / 32) : 1e12;
     std::string key(reinterpret_cast<const char*>(&g), sizeof(Geom));
     key.append(reinterpret_cast<const char*>(&cap_z), sizeof(int));
     {
         std::lock_guard<std::mutex> lk(mu);
         auto it = cache.find(key);
-        if (it != cache.end()) return it->second;
+        if (it != cache.end()) {
+            int R = it->second.base.R, NW = it->second.base.NW;
+            cell_shape(g.Nv, it->second.base.fine, grid, R, NW);
+            for (size_t i = 0; i < it->second.asked.size(); ++i)
+                if (it->second.asked[i] == std::make_pair(R, NW)) return it->second.shapes[i];
+        }
     }
     double coarse = 0.0, wide = 0.0, pairs = 0.0;
     const double uscale = (g.type == GEO_FLAT) ? g.sod / g.sdd : 1.0;
@@ -322,7 +341,8 @@ CellPlans plan_cell_shapes(const Geom& g, int cap_z) {
     CellPlans r;
     r.base = make(cell_rows_per_thread(g), CELL_NW);
     int R = r.base.R, NW = r.base.NW;
-    cell_shape(g.Nv, fine, R, NW);
+    cell_shape(g.Nv, fine, grid, R, NW);
+    const std::pair<int, int> asked{R, NW};
     r.launch = R == r.base.R && NW == r.base.NW ? r.base : make(R, NW);
     // the default shape where the other's windows leave an SM fewer warps (its
     // registers allow 16)
@@ -332,11 +352,16 @@ CellPlans plan_cell_shapes(const Geom& g, int cap_z) {
     };
     if (!r.launch.ok || warps(r.launch) < std::min(12, warps(r.base))) r.launch = r.base;
     std::lock_guard<std::mutex> lk(mu);
-    cache[key] = r;
+    Known& k = cache[key];
+    k.base = r.base;
+    if (std::find(k.asked.begin(), k.asked.end(), asked) == k.asked.end()) {
+        k.asked.push_back(asked);
+        k.shapes.push_back(r);
+    }
     return r;
 }
 
-CellPlan plan_cell(const Geom& g) { return plan_cell_shapes(g, 1 << 30).base; }
+CellPlan plan_cell(const Geom& g) { return plan_cell_shapes(g, 1 << 30, 0).base; }
 
 using EncodeTiledFn = PFN_cuTensorMapEncodeTiled_v12000;
 
@@ -806,11 +831,11 @@ int launch_cell_tma_mode(const Geom& g, const CellPlan& p, const CUtensorMap& mr
 // Window plan of a helical scan: the views' z placement varies, so the z
 // extent is sized on a volume deep enough that no window is clamped, then
 // capped at the real depth (a window never spans more than D + 2 slices).
-CellPlans plan_cell_helical(const Geom& g) {
+CellPlans plan_cell_helical(const Geom& g, long long images) {
     Geom gp = g;
     gp.D = 1 << 20;
     gp.shz = 0.0;
-    return plan_cell_shapes(gp, g.D + 2);
+    return plan_cell_shapes(gp, g.D + 2, images);
 }
 
 // The unstaged gather; CS: the split that the staged one would take, followed
@@ -833,7 +858,8 @@ int run_cell_tma(int eff, const Geom& g, const float* in, TO* out, int nbatch, i
                  const float* zwt = nullptr) {
     using TI = float;  // half-precision images are widened first
     if (reinterpret_cast<uintptr_t>(in) % 16 != 0) return -1;
-    const CellPlans plans = HEL ? plan_cell_helical(g) : plan_cell_shapes(g, 1 << 30);
+    const long long images = (long long)nview * nbatch;
+    const CellPlans plans = HEL ? plan_cell_helical(g, images) : plan_cell_shapes(g, 1 << 30, images);
     if (!plans.base.ok || !encode_fn()) return -1;
     const CellPlan& p = plans.launch;
     const size_t es = sizeof(TI);
@@ -1626,11 +1652,11 @@ int xr_cell_plan(const xr_geom3d* geom, int* ok, int* box_pixels, int* box_z, in
     return XR_OK;
 }
 
-int xr_cell_launch_plan(const xr_geom3d* geom, int* rows_per_thread, int* warps, int* pixels) {
+int xr_cell_launch_plan(const xr_geom3d* geom, int nbatch, int nview, int* rows_per_thread, int* warps, int* pixels) {
     if (!geom || !rows_per_thread || !warps || !pixels) return xr::fail(XR_ERR_INVALID_ARGUMENT, "null pointer");
     const xr::Geom g = xr::geom_from(geom);
-    if (int rc = xr::validate(g, 1, 0, 1, 1)) return rc;
-    const xr::CellPlans p = xr::plan_cell_shapes(g, 1 << 30);
+    if (int rc = xr::validate(g, 1, 0, nbatch, nview)) return rc;
+    const xr::CellPlans p = xr::plan_cell_shapes(g, 1 << 30, (long long)nbatch * nview);
     *rows_per_thread = p.base.ok ? p.launch.R : 0;
     *warps = p.base.ok ? p.launch.NW : 0;
     *pixels = p.base.ok ? (p.launch.fine ? p.launch.NB : 2) : 0;
